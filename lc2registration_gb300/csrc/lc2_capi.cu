@@ -1579,6 +1579,7 @@ int set_static_bins(lc2_context* c) {
 // fmax: the fixed image's largest |value| (image_absmax).
 int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
   const int storage = c->cfg.storage;
+  drop_graphs(c);  // they hold the old images' fixed-point scales
   struct Free {
     float* p;
     cudaStream_t st;
