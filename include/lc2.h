@@ -155,10 +155,9 @@ long long lc2_launch_count(const lc2_context* ctx);
 
 /* Tuning options (lc2_set_option). LC2_OPTION_TILE_ROWS: output rows per
  * tile of the fused 3D kernels at patch radius 1-4: 16 (one 512-thread CTA
- * per SM), 24 (one 768-thread CTA per SM; on presampled images, and for a
- * resampled MR/CT resampled in the kernel; elsewhere taken as 16; a grid
- * whose height leaves 1-16 rows over runs them on 16-row tiles) or 8 (two
- * CTAs per SM); radius 5-6 always runs 8. 0 = automatic: 24 on presampled
+ * per SM), 24 (one CTA per SM; on presampled images, and for a resampled
+ * MR/CT resampled in the kernel; elsewhere taken as 16; a grid whose height
+ * leaves 1-16 rows over runs them on 16-row tiles) or 8 (two CTAs per SM); radius 5-6 always runs 8. 0 = automatic: 24 on presampled
  * images -- of a resampled MR/CT on any grid, of a resampled ultrasound on
  * grids of 8 M voxels or more -- and for a resampled MR/CT at radius 3 or 4
  * when the kernel resamples itself (LC2_OPTION_PRESAMPLE 0); else 16. 2D and
@@ -203,7 +202,7 @@ enum { LC2_OPTION_GENERIC = 7 };
 /* LC2_OPTION_PRESAMPLE (3D, HighResolutionModality Moving): how the moving
  * image is resampled. 1 (the default of such contexts): in a pass of its own,
  * one float per virtual voxel and transform written to a context buffer that
- * grows with the batch up to 2 GiB (32 transforms at 256^3; larger batches
+ * grows with the batch up to 2 GiB (26 transforms at 256^3; larger batches
  * run in groups), which the fused kernel then reads; 0: inside the fused
  * kernel. Other values are refused (LC2_ERR_INVALID_ARGUMENT). Each voxel is
  * sampled once from its 32 x 8 tile's base in form 1 and from the fused

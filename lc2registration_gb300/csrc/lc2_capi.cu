@@ -19,6 +19,7 @@
 #include "lc2_fused.cuh"
 #include "lc2_fused_fixed.cuh"
 #include "lc2_fused_ps.cuh"
+#include "lc2_quad.cuh"
 #include "lc2_list.cuh"
 #include "lc2_mi.cuh"
 
@@ -223,6 +224,13 @@ struct lc2_context {
   int presample = 0;  // 3D: resample as a pass of its own (LC2_OPTION_PRESAMPLE)
   float* d_pre = nullptr;  // presampled images (FP32 M) of pre_slots transforms
   int pre_slots = 0;
+  bool pre_padded = false;  // d_pre holds images of the padded layout (zero borders)
+  // 3D resampled MR/CT at radius <= 4: the padded layout of k_fused_quad and
+  // the quantised static ultrasound in it
+  bool quad = false;
+  lc2::PadLayout lay{};
+  int* d_uq = nullptr;
+  int2* d_ss = nullptr;  // its weighting factor (float bits) and window sum, padded too
   int* d_err = nullptr;   // device flag of the warp-specialised kernel's bounded waits
   int* h_err = nullptr;   // pinned copy
 
@@ -277,6 +285,21 @@ __global__ void k_box_line(const T* __restrict__ in, T* __restrict__ out, int nx
     if (i + r < len) a += in[base + (size_t)(i + r) * stride];
     if (i - r - 1 >= 0) a -= in[base + (size_t)(i - r - 1) * stride];
     out[base + (size_t)i * stride] = a;
+  }
+}
+
+// The static ultrasound's fields in padded strides: quantised values, and
+// (weighting factor bits, window sum) pairs.
+template <typename TU>
+__global__ void k_pad_static(const TU* __restrict__ U, float qu, const float* __restrict__ sig,
+                             const int* __restrict__ su, int nx, int ny, size_t n,
+                             int* __restrict__ uq, int2* __restrict__ ss, int row, size_t plane) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t l = i / nx, z = l / ny;
+    const size_t o = z * plane + (l - z * ny) * row + (i - l * nx);
+    uq[o] = quant(ldf(U, i), qu);
+    ss[o] = make_int2(__float_as_int(sig[i]), su[i]);
   }
 }
 
@@ -635,8 +658,8 @@ int launch_group_generic(lc2_context* c, int k0, int cnt, float* osig, float* om
 
 // Output rows per tile of the fused kernels: the option if set; in 2D 0 (per
 // launch); in 3D at patch radius 1-4, 24 -- on presampled images of a
-// resampled MR/CT (k_fused_pt: batched 4-14 % faster than 16-row tiles from
-// 48^3 to 256^3 grids, one transform per call up to 15 %), on a presampled
+// resampled MR/CT (k_fused_quad, with 16-row tiles of its own for the rows
+// that 24-row tiles leave over), on a presampled
 // ultrasound for grids of 8 M voxels or more (k_fused_fixed_pt: at 256^3
 // 1.4 % batched and 5 % per call; on 48^3 to 160^3 grids 16 rows were up to
 // 3 % faster), and for a resampled MR/CT resampled in the kernel at radius 3
@@ -652,24 +675,65 @@ int tile_rows(const lc2_context* c) {
 
 // The fused kernel (static ultrasound): one launch for `cnt` transforms.
 // The presample buffer holds the images of a group of transforms, at most
-// 2 GiB and 64 transforms -- 32 at 256^3. It grows with the batches a context is
+// 2 GiB and 64 transforms -- 26 padded ones at 256^3. It grows with the batches a context is
 // given (a registration's single evaluations hold one slot); growing moves
 // it, which drops the captured graphs that name it.
 constexpr size_t kPresampleBytes = size_t(2) << 30;
-int presample_cap(const lc2_context* c) {
-  const size_t per = sizeof(float) * c->nv;
+
+// Whether the context's batches run on k_fused_quad: presampled images of a
+// resampled MR/CT at radius <= 4, unless 8- or 16-row tiles are asked for.
+bool use_quad(const lc2_context* c) {
+  return c->quad && c->presample && !c->pipeline && tile_rows(c) == 24;
+}
+
+// Voxels of one presampled image in the layout in use.
+size_t presample_voxels(const lc2_context* c, bool padded) {
+  return padded ? c->lay.volume() : c->nv;
+}
+
+int presample_cap(const lc2_context* c, bool padded) {
+  const size_t per = sizeof(float) * presample_voxels(c, padded);
   return (int)std::max<size_t>(1, std::min<size_t>(64, kPresampleBytes / per));
 }
 
+// The padded layout's borders are zeroed once, here: k_presample writes the
+// voxels of the grid only.
 int ensure_presample(lc2_context* c, int count) {
-  const int want = std::max(1, std::min(count, presample_cap(c)));
-  if (c->d_pre && c->pre_slots >= want) return LC2_OK;
+  const bool padded = use_quad(c);
+  const int want = std::max(1, std::min(count, presample_cap(c, padded)));
+  if (c->d_pre && c->pre_slots >= want && c->pre_padded == padded) return LC2_OK;
   drop_graphs(c);
   dev_free(c->d_pre, c->stream);
   c->d_pre = nullptr;
   c->pre_slots = 0;
-  LC2_CUDA(dev_alloc((void**)&c->d_pre, sizeof(float) * c->nv * (size_t)want, c->stream));
+  const size_t bytes = sizeof(float) * presample_voxels(c, padded) * (size_t)want;
+  LC2_CUDA(dev_alloc((void**)&c->d_pre, bytes, c->stream));
+  if (padded) LC2_CUDA(cudaMemsetAsync(c->d_pre, 0, bytes, c->stream));
   c->pre_slots = want;
+  c->pre_padded = padded;
+  return LC2_OK;
+}
+
+// k_presample of transforms [k0, k0 + n) into the presample buffer.
+int launch_presample(lc2_context* c, int k0, int n) {
+  const bool padded = c->pre_padded;
+  const int row = padded ? c->lay.px : c->virt.dim[0];
+  const size_t plane = padded ? c->lay.slice() : (size_t)c->virt.dim[0] * c->virt.dim[1];
+  const size_t volume = presample_voxels(c, padded);
+  float* out = c->d_pre + (padded ? c->lay.first() + c->lay.origin() : 0);
+  TimerScope ts(c, K_WARP);
+  cudaError_t e;
+  if (c->cfg.storage == LC2_STORE_F16)
+    e = lc2::presample_launch<__half>(c->d_moving, c->fp, c->d_xf, k0, n, out, row, plane, volume,
+                                      c->stream);
+  else if (c->cfg.storage == LC2_STORE_BF16)
+    e = lc2::presample_launch<__nv_bfloat16>(c->d_moving, c->fp, c->d_xf, k0, n, out, row, plane,
+                                             volume, c->stream);
+  else
+    e = lc2::presample_launch<float>(c->d_moving, c->fp, c->d_xf, k0, n, out, row, plane, volume,
+                                     c->stream);
+  ++c->launches;
+  LC2_CUDA(e);
   return LC2_OK;
 }
 
@@ -758,23 +822,17 @@ int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
     // resample pass, then the fused kernel on the presampled images, in
     // groups of the presample buffer's capacity
     LC2_TRY(ensure_presample(c, cnt));
-    auto presample = [&](int j, int n, float* buf) {
-      const cudaStream_t st = c->stream;
-      if (c->cfg.storage == LC2_STORE_F16)
-        return lc2::presample_launch<__half>(c->d_moving, c->fp, c->d_xf, k0 + j, n, buf, st);
-      if (c->cfg.storage == LC2_STORE_BF16)
-        return lc2::presample_launch<__nv_bfloat16>(c->d_moving, c->fp, c->d_xf, k0 + j, n, buf,
-                                                    st);
-      return lc2::presample_launch<float>(c->d_moving, c->fp, c->d_xf, k0 + j, n, buf, st);
-    };
+    const bool quad = use_quad(c);
     auto moments_one = [&](const float* buf) {
+      if (quad) return lc2::quad_launch(L, buf, c->d_uq, c->d_ss, c->lay);
       if (c->cfg.storage == LC2_STORE_F16) return lc2::fused_ps_entry<__half>(L, buf);
       if (c->cfg.storage == LC2_STORE_BF16) return lc2::fused_ps_entry<__nv_bfloat16>(L, buf);
       return lc2::fused_ps_entry<float>(L, buf);
     };
     // the moments pass of a group: radius <= 4 with the in-kernel Sobel
-    // (k_fused_pt on 24-row tiles, the rows left over by them as one row
-    // of k_fused_ps tiles; k_fused_ps on 8/16-row tiles), else k_fused
+    // (k_fused_quad on 24-row tiles, the rows left over by them as one row of
+    // its 16-row tiles; k_fused_ps where 8/16-row tiles are asked for), else
+    // k_fused
     auto moments = [&](int j, int n, const float* buf) {
       L.k0 = k0 + j;
       L.cnt = n;
@@ -799,18 +857,13 @@ int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
       L.y_off = L.y_rows = 0;
       return err;
     };
-    // the moments kernel's tile height: 24 (k_fused_pt), 16 (k_fused_ps) or,
+    // the moments kernel's tile height: 24 (k_fused_quad), 16 (k_fused_ps) or,
     // beyond radius 4, 8 (k_fused on presampled images)
     const int ty = c->cfg.patch_size > 4 ? 8 : (L.tile_height == 24 ? 24 : 16);
     const int group = presample_group(c, cnt, ty, 1);
     for (int j = 0; j < cnt; j += group) {
       const int n = std::min(group, cnt - j);
-      {
-        TimerScope ts(c, K_WARP);
-        e = presample(j, n, c->d_pre);
-      }
-      ++c->launches;
-      LC2_CUDA(e);
+      LC2_TRY(launch_presample(c, k0 + j, n));
       {
         TimerScope ts(c, K_MOMENTS);
         e = moments(j, n, c->d_pre);
@@ -878,18 +931,7 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
     const int rest = ty == 24 ? pt_rest_rows(c) : 0;
     for (int j = 0; j < cnt; j += group) {
       const int n = std::min(group, cnt - j);
-      {
-        TimerScope ts(c, K_WARP);
-        if (c->cfg.storage == LC2_STORE_F16)
-          e = lc2::presample_launch<__half>(c->d_moving, c->fp, c->d_xf, k0 + j, n, c->d_pre, c->stream);
-        else if (c->cfg.storage == LC2_STORE_BF16)
-          e = lc2::presample_launch<__nv_bfloat16>(c->d_moving, c->fp, c->d_xf, k0 + j, n, c->d_pre,
-                                                   c->stream);
-        else
-          e = lc2::presample_launch<float>(c->d_moving, c->fp, c->d_xf, k0 + j, n, c->d_pre, c->stream);
-      }
-      ++c->launches;
-      LC2_CUDA(e);
+      LC2_TRY(launch_presample(c, k0 + j, n));
       L.k0 = k0 + j;
       L.cnt = n;
       L.pre = c->d_pre;
@@ -1095,6 +1137,11 @@ int plan_context(const lc2_config* cfg, lc2_context* c) {
   c->slots = (int)std::max<long long>(1, slots);
   // 3D contexts of a resampled MR/CT resample in a pass of their own
   c->presample = (c->lc2_nd == 3 && !c->mi) ? 1 : 0;
+  // the padded images of k_fused_quad index a slice with 32-bit byte offsets
+  if (c->presample && cfg->high_res_is_moving && r <= 4) {
+    c->lay = lc2::pad_layout(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], r);
+    c->quad = c->lay.slice() < (size_t)1 << 29;
+  }
   return LC2_OK;
 }
 
@@ -1114,7 +1161,9 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
     h += c->nv + 64 * (sizeof(unsigned) * (lc2::kMiHist + 2) + sizeof(double) * 2 * lc2::kMiParts);
   h += 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
   if (c->presample)  // the presample buffer at its largest
-    h += sizeof(float) * c->nv * (size_t)presample_cap(c);
+    h += sizeof(float) * std::max(presample_voxels(c, c->quad) * (size_t)presample_cap(c, c->quad),
+                                  c->nv * (size_t)presample_cap(c, false));
+  if (c->quad) h += (sizeof(int) + sizeof(int2)) * c->lay.volume();  // padded static fields
   *held = h;
   *peak_extra = std::max(c->nm, c->nf) * sizeof(float);
   if (!hrm && !c->mi)  // temporaries of the static sums
@@ -1153,6 +1202,10 @@ int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
     e = dev_alloc((void**)&c->d_sigma, c->nv * sizeof(float), c->stream);
   if (e == cudaSuccess && cfg->high_res_is_moving && !c->mi)
     e = dev_alloc((void**)&c->d_su, c->nv * sizeof(int), c->stream);
+  if (e == cudaSuccess && c->quad)
+    e = dev_alloc((void**)&c->d_uq, c->lay.volume() * sizeof(int), c->stream);
+  if (e == cudaSuccess && c->quad)
+    e = dev_alloc((void**)&c->d_ss, c->lay.volume() * sizeof(int2), c->stream);
   if (e == cudaSuccess && c->mi) e = dev_alloc((void**)&c->d_sbin, c->nv, c->stream);
   if (e == cudaSuccess && !cfg->high_res_is_moving && !c->mi)
     e = dev_alloc((void**)&c->d_fq, 2 * c->nv * sizeof(int), c->stream);
@@ -1216,6 +1269,8 @@ int lc2_destroy(lc2_context* c) {
   dev_free(c->d_sigma, fs);
   dev_free(c->d_su, fs);
   dev_free(c->d_pre, fs);
+  dev_free(c->d_uq, fs);
+  dev_free(c->d_ss, fs);
   dev_free(c->d_fq, fs);
   dev_free(c->d_fs, fs);
   dev_free(c->d_fd, fs);
@@ -1473,6 +1528,23 @@ int static_window_sum(lc2_context* c) {
     pass(tb, c->d_su, 1, (long long)nx * nz);
   }
   c->launches += (c->lc2_nd == 3) ? 4 : 3;
+  if (c->quad) {
+    const size_t at = c->lay.first() + c->lay.origin();
+    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.volume() * sizeof(int), c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.volume() * sizeof(int2), c->stream));
+    auto pad = [&](auto* u) {
+      lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(u, c->fp.qu, c->d_sigma, c->d_su, nx, ny, nv,
+                                                       c->d_uq + at, c->d_ss + at, c->lay.px,
+                                                       c->lay.slice());
+    };
+    if (st == LC2_STORE_F16)
+      pad((const __half*)c->d_static);
+    else if (st == LC2_STORE_BF16)
+      pad((const __nv_bfloat16*)c->d_static);
+    else
+      pad((const float*)c->d_static);
+    ++c->launches;
+  }
   LC2_CUDA(cudaGetLastError());
   LC2_CUDA(cudaStreamSynchronize(c->stream));
   return LC2_OK;

@@ -595,14 +595,16 @@ constexpr int fused_min_blocks(int nd, int ty, int r) {
 // bases are computed by 3 kPreZ threads at once, and each thread then has
 // kPreZ independent samples in flight. The output is written with streaming
 // stores (it is read once, by another kernel, and should not evict the
-// moving volume from L2).
+// moving volume from L2). out: voxel (0, 0, 0) of the first image; row, plane
+// and volume: its strides.
 constexpr int kPreZ = 8;
 
 template <typename TM>
 __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, int mx, int my,
                                                    int mz, int vx, int vy, int vz,
                                                    const Xform* __restrict__ xf, int k0,
-                                                   float* __restrict__ out) {
+                                                   float* __restrict__ out, int row,
+                                                   size_t plane, size_t volume) {
   __shared__ int s_ib[kPreZ][3];
   __shared__ float s_fb[kPreZ][3];
   __shared__ float s_A[9];
@@ -634,8 +636,7 @@ __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, i
   const int tx = tid & 31, ty = tid >> 5;
   const int x = x0 + tx, y = y0 + ty;
   if (x >= vx || y >= vy) return;
-  const size_t plane = (size_t)vx * vy;
-  float* dst = out + (size_t)slot * plane * vz + (size_t)y * vx + x;
+  float* dst = out + (size_t)slot * volume + (size_t)y * row + x;
   float v[kPreZ];
 #pragma unroll
   for (int zs = 0; zs < kPreZ; ++zs) {
@@ -1029,14 +1030,15 @@ cudaError_t fused_launch_grid(const FusedLaunch& L, K kern) {
   return cudaGetLastError();
 }
 
-// k_presample of transforms [k0, k0 + cnt) into pre (cnt x voxels floats).
+// k_presample of transforms [k0, k0 + cnt) into images of these strides.
 template <typename T>
 cudaError_t presample_launch(const void* mov, const FusedParams& P, const Xform* xf, int k0,
-                             int cnt, float* pre, cudaStream_t stream) {
+                             int cnt, float* pre, int row, size_t plane, size_t volume,
+                             cudaStream_t stream) {
   const int ntx = (P.vx + 31) / 32, nty = (P.vy + 7) / 8;
   dim3 grid(ntx * nty, (P.vz + kPreZ - 1) / kPreZ, cnt);
   k_presample<T><<<grid, 256, 0, stream>>>((const T*)mov, P.mx, P.my, P.mz, P.vx, P.vy, P.vz, xf,
-                                           k0, pre);
+                                           k0, pre, row, plane, volume);
   return cudaGetLastError();
 }
 
