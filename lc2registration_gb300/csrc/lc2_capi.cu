@@ -20,6 +20,7 @@
 #include "lc2_fused_fixed.cuh"
 #include "lc2_fused_ps.cuh"
 #include "lc2_quad.cuh"
+#include "lc2_quad_fixed.cuh"
 #include "lc2_list.cuh"
 #include "lc2_mi.cuh"
 
@@ -225,8 +226,9 @@ struct lc2_context {
   float* d_pre = nullptr;  // presampled images (FP32 M) of pre_slots transforms
   int pre_slots = 0;
   bool pre_padded = false;  // d_pre holds images of the padded layout (zero borders)
-  // 3D resampled MR/CT at radius <= 4: the padded layout of k_fused_quad and
-  // the quantised static ultrasound in it
+  // 3D at radius <= 4: the padded layout of k_fused_quad / k_fixed_quad and in
+  // it the quantised static ultrasound or (resampled ultrasound) the quantised
+  // static image and its Sobel magnitude, one after the other
   bool quad = false;
   lc2::PadLayout lay{};
   int* d_uq = nullptr;
@@ -285,6 +287,16 @@ __global__ void k_box_line(const T* __restrict__ in, T* __restrict__ out, int nx
     if (i + r < len) a += in[base + (size_t)(i + r) * stride];
     if (i - r - 1 >= 0) a -= in[base + (size_t)(i - r - 1) * stride];
     out[base + (size_t)i * stride] = a;
+  }
+}
+
+// An image of rows nx and ny rows per slice into padded strides.
+__global__ void k_pad(const int* __restrict__ in, int nx, int ny, size_t n, int* __restrict__ out,
+                      int row, size_t plane) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t l = i / nx, z = l / ny;
+    out[z * plane + (l - z * ny) * row + (i - l * nx)] = in[i];
   }
 }
 
@@ -657,19 +669,16 @@ int launch_group_generic(lc2_context* c, int k0, int cnt, float* osig, float* om
 }
 
 // Output rows per tile of the fused kernels: the option if set; in 2D 0 (per
-// launch); in 3D at patch radius 1-4, 24 -- on presampled images of a
-// resampled MR/CT (k_fused_quad, with 16-row tiles of its own for the rows
-// that 24-row tiles leave over), on a presampled
-// ultrasound for grids of 8 M voxels or more (k_fused_fixed_pt: at 256^3
-// 1.4 % batched and 5 % per call; on 48^3 to 160^3 grids 16 rows were up to
-// 3 % faster), and for a resampled MR/CT resampled in the kernel at radius 3
-// or 4 (one 768-thread CTA per SM) -- else 16.
+// launch); in 3D at patch radius 1-4, 24 on presampled images (k_fused_quad and
+// k_fixed_quad, with 16-row tiles of their own for the rows that 24-row tiles
+// leave over) and for a resampled MR/CT resampled in the kernel at radius 3 or
+// 4 (one 768-thread CTA per SM), else 16.
 int tile_rows(const lc2_context* c) {
   if (c->tile_rows > 0) return c->tile_rows;
   if (c->lc2_nd == 2) return 0;  // chosen per launch: 32 rows for large launches, else 16
   const int r = c->cfg.patch_size;
   if (c->lc2_nd != 3 || r > 4) return 16;
-  if (c->presample) return (c->cfg.high_res_is_moving || c->nv >= 8000000) ? 24 : 16;
+  if (c->presample && c->quad) return 24;
   return (c->cfg.high_res_is_moving && r >= 3) ? 24 : 16;
 }
 
@@ -680,10 +689,11 @@ int tile_rows(const lc2_context* c) {
 // it, which drops the captured graphs that name it.
 constexpr size_t kPresampleBytes = size_t(2) << 30;
 
-// Whether the context's batches run on k_fused_quad: presampled images of a
-// resampled MR/CT at radius <= 4, unless 8- or 16-row tiles are asked for.
+// Whether the context's batches run on k_fused_quad or k_fixed_quad: presampled
+// images at radius <= 4, unless 8- or 16-row tiles are asked for.
 bool use_quad(const lc2_context* c) {
-  return c->quad && c->presample && !c->pipeline && tile_rows(c) == 24;
+  return c->quad && c->presample && !(c->pipeline && c->cfg.high_res_is_moving) &&
+         tile_rows(c) == 24;
 }
 
 // Voxels of one presampled image in the layout in use.
@@ -909,6 +919,7 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
   L.stream = c->stream;
   auto fixed = [&]() {
     TimerScope ts(c, K_MOMENTS);
+    if (use_quad(c)) return lc2::fixed_quad_launch(L, c->d_uq, c->lay);
     switch (c->cfg.storage) {
       case LC2_STORE_F16: return lc2::fixed_launch<__half>(L);
       case LC2_STORE_BF16: return lc2::fixed_launch<__nv_bfloat16>(L);
@@ -921,7 +932,7 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
     // groups of the presample buffer's capacity
     LC2_TRY(ensure_presample(c, cnt));
     // the moments kernel's tile height and CTAs per SM: 24 rows
-    // (k_fused_fixed_pt, the rows it leaves over on 16-row tiles), else
+    // (k_fixed_quad, the rows it leaves over on its 16-row tiles), else
     // k_fused_fixed3's 16 or 8
     const int ty = c->cfg.patch_size > 4 || L.tile_height == 8 ? 8
                    : L.tile_height == 24                       ? 24
@@ -1138,7 +1149,7 @@ int plan_context(const lc2_config* cfg, lc2_context* c) {
   // 3D contexts of a resampled MR/CT resample in a pass of their own
   c->presample = (c->lc2_nd == 3 && !c->mi) ? 1 : 0;
   // the padded images of k_fused_quad index a slice with 32-bit byte offsets
-  if (c->presample && cfg->high_res_is_moving && r <= 4) {
+  if (c->presample && r <= 4) {
     c->lay = lc2::pad_layout(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], r);
     c->quad = c->lay.slice() < (size_t)1 << 29;
   }
@@ -1163,7 +1174,8 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
   if (c->presample)  // the presample buffer at its largest
     h += sizeof(float) * std::max(presample_voxels(c, c->quad) * (size_t)presample_cap(c, c->quad),
                                   c->nv * (size_t)presample_cap(c, false));
-  if (c->quad) h += (sizeof(int) + sizeof(int2)) * c->lay.volume();  // padded static fields
+  // padded static fields: quantised ultrasound and its (sigma, S_U), or M and G
+  if (c->quad) h += (hrm ? sizeof(int) + sizeof(int2) : 2 * sizeof(int)) * c->lay.volume();
   *held = h;
   *peak_extra = std::max(c->nm, c->nf) * sizeof(float);
   if (!hrm && !c->mi)  // temporaries of the static sums
@@ -1203,8 +1215,9 @@ int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
   if (e == cudaSuccess && cfg->high_res_is_moving && !c->mi)
     e = dev_alloc((void**)&c->d_su, c->nv * sizeof(int), c->stream);
   if (e == cudaSuccess && c->quad)
-    e = dev_alloc((void**)&c->d_uq, c->lay.volume() * sizeof(int), c->stream);
-  if (e == cudaSuccess && c->quad)
+    e = dev_alloc((void**)&c->d_uq,
+                  c->lay.volume() * (cfg->high_res_is_moving ? 1 : 2) * sizeof(int), c->stream);
+  if (e == cudaSuccess && c->quad && cfg->high_res_is_moving)
     e = dev_alloc((void**)&c->d_ss, c->lay.volume() * sizeof(int2), c->stream);
   if (e == cudaSuccess && c->mi) e = dev_alloc((void**)&c->d_sbin, c->nv, c->stream);
   if (e == cudaSuccess && !cfg->high_res_is_moving && !c->mi)
@@ -1569,6 +1582,15 @@ int fixed_static_sums(lc2_context* c) {
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
   lc2::k_fixed_quant<<<blocks, 256, 0, c->stream>>>((const float*)c->d_static, c->d_gstatic, nv,
                                                     c->fp.qm, c->fp.qg, c->d_fq, c->d_fd);
+  if (c->quad) {
+    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, 2 * c->lay.volume() * sizeof(int), c->stream));
+    for (int f = 0; f < 2; ++f)
+      lc2::k_pad<<<blocks, 256, 0, c->stream>>>(
+          c->d_fq + f * nv, nx, ny, nv,
+          c->d_uq + f * c->lay.volume() + c->lay.first() + c->lay.origin(), c->lay.px,
+          c->lay.slice());
+    c->launches += 2;
+  }
   auto pass = [&](auto* in, auto* out, int axis) {
     const long long lines = axis == 0 ? (long long)ny * nz : axis == 1 ? (long long)nx * nz
                                                                        : (long long)nx * ny;
@@ -1820,7 +1842,8 @@ namespace {
 int stage_host(lc2_context* c, const float* matrices, int count) {
   if (count < 0 || (count > 0 && !matrices)) return fail(LC2_ERR_INVALID_ARGUMENT, "bad transforms");
   LC2_TRY(ensure_capacity(c, count));
-  if (c->presample && !c->generic && !c->pipeline) LC2_TRY(ensure_presample(c, count));
+  if (c->presample && !c->generic && !(c->pipeline && c->cfg.high_res_is_moving))
+    LC2_TRY(ensure_presample(c, count));
   const int mf = matrix_floats(c);
   for (int k = 0; k < count; ++k) {
     const float* m = matrices + (size_t)k * mf;

@@ -77,9 +77,11 @@ struct QuadParams {
 // (8.1), the Sobel magnitudes as a pass of their own (7.5 and 0.7 for the pass).
 constexpr int kQuadOut = 4;  // output rows per solving thread
 
-template <int TY, int R>
+// NL limb planes; NRING 16-byte ring entries per moments thread and slice of
+// the window; SOBEL: the (Sz, Dz) planes of a resampled MR/CT.
+template <int TY, int R, int NL = kLimbs, int NRING = 1, bool SOBEL = true>
 struct QuadGeom {
-  static constexpr int W = 2 * R + 1;
+  static constexpr int R_ = R, W = 2 * R + 1;
   static constexpr int HX = 32 + 2 * R, HY = TY + 2 * R;
   static constexpr int NQ = (HY + 3) / 4;                     // halo quads per column
   static constexpr int TAIL = 2 * R * NQ;                     // threads of the columns beyond 32
@@ -88,8 +90,10 @@ struct QuadGeom {
   static constexpr int CT = 32 * (TY / kQuadOut);             // window / solve threads
   static constexpr int NT = PT + CT;
   // x pass: jobs (limb, quad of rows), their 32 output columns in XP parts
-  static constexpr int XJOBS = kLimbs * NQ;
-  static constexpr int XP = CT / XJOBS > 0 ? CT / XJOBS : 1, XC = (32 + XP - 1) / XP;
+  static constexpr int XJOBS = NL * NQ;
+  static constexpr int XT = SOBEL ? CT : PT;                  // threads that run the x pass
+  static constexpr int XP = XT / XJOBS > 3 ? 3 : XT / XJOBS > 0 ? XT / XJOBS : 1;
+  static constexpr int XC = (32 + XP - 1) / XP;
   // (Sz, Dz) planes: the halo with a one-voxel margin. Pitch = 2 mod 4 float2,
   // so that the 8-column tail's four quads of a warp (rows 4 apart) read
   // distinct banks.
@@ -103,14 +107,15 @@ struct QuadGeom {
   static constexpr int PA = HX * YP + (32 + 4 * (NQ % 8) - HX * YP % 32) % 32;
   static constexpr int PY = 32 * YP + (32 + 4 * (NQ % 8) - 32 * YP % 32) % 32;
   static constexpr int RING = 2 * R + 1;
-  static constexpr size_t OFF_SD = sizeof(int4) * (size_t)RING * PT;           // after the ring
-  static constexpr size_t OFF_A = OFF_SD + sizeof(float2) * 2 * (size_t)SP * SR;
-  static constexpr size_t OFF_Y = OFF_A + sizeof(int) * (size_t)kLimbs * PA;
-  static constexpr size_t BYTES = OFF_Y + sizeof(int) * (size_t)kLimbs * PY;
+  static constexpr size_t OFF_SD = sizeof(int4) * (size_t)NRING * RING * PT;  // after the ring
+  static constexpr size_t OFF_A = OFF_SD + (SOBEL ? sizeof(float2) * 2 * (size_t)SP * SR : 0);
+  static constexpr size_t OFF_Y = OFF_A + sizeof(int) * (size_t)NL * PA;
+  static constexpr size_t BYTES = OFF_Y + sizeof(int) * (size_t)NL * PY;
   static constexpr int NV = (kQuadOut + W - 1 + 3) / 4;       // quads a solving thread reads
   static_assert(SP % 4 == 2 && SP >= HX + 2 && OFF_A % 16 == 0 && PA % 4 == 0 && PY % 4 == 0, "");
   static_assert(TY % kQuadOut == 0 && TY / 4 - kQuadOut / 4 + NV <= NQ, "a solve stays in the plane");
   static_assert(NM <= PT, "one margin point per moments thread");
+  static_assert(XJOBS <= XT, "every x job has a thread");
   static_assert(BYTES <= 227 * 1024, "one CTA's shared memory must fit an SM");
 };
 
@@ -148,9 +153,8 @@ __device__ __forceinline__ float div_ftz(float a, float b) {
 
 // Window sums of one limb at kQuadOut consecutive rows: o[j] = sum of rows
 // j .. j + 2R of the column at y.
-template <int TY, int R>
+template <typename G>
 __device__ __forceinline__ void quad_window(const int* __restrict__ y, int* o) {
-  using G = QuadGeom<TY, R>;
   int v[4 * G::NV];
 #pragma unroll
   for (int i = 0; i < G::NV; ++i) {
@@ -174,18 +178,44 @@ __device__ __forceinline__ void quad_window(const int* __restrict__ y, int* o) {
 // Centred sums D = n S - a b of kQuadOut outputs, S = hi 2^K + lo from the
 // window sums of limb planes L (lo) and L + 1 (hi); n 2^K fits 31 bits by the
 // choice of K.
-template <int TY, int R>
+template <typename G>
 __device__ __forceinline__ void quad_centred(const int* __restrict__ y, int L, const int* a,
                                              const int* b, long long* d) {
-  using G = QuadGeom<TY, R>;
-  using C = PatchConst<3, R>;
+  using C = PatchConst<3, G::R_>;
   constexpr int n = (int)C::N, nk = (int)(C::N << C::K);
   int lo[kQuadOut], hi[kQuadOut];
-  quad_window<TY, R>(y + (size_t)L * G::PY, lo);
-  quad_window<TY, R>(y + (size_t)(L + 1) * G::PY, hi);
+  quad_window<G>(y + (size_t)L * G::PY, lo);
+  quad_window<G>(y + (size_t)(L + 1) * G::PY, hi);
 #pragma unroll
   for (int j = 0; j < kQuadOut; ++j)
     d[j] = (long long)hi[j] * nk + (long long)lo[j] * n - (long long)a[j] * b[j];
+}
+
+// x window pass from the limb planes to Y: four rows of one limb per thread, a
+// running sum along XC + 2R columns.
+template <typename G>
+__device__ __forceinline__ void quad_xpass(bool job, const int* __restrict__ a,
+                                           int* __restrict__ y) {
+  if (G::XP * G::XJOBS == G::XT || job) {
+    int4 v[G::XC + G::W - 1];
+    int4 w = make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < G::XC + G::W - 1; ++i) {
+      v[i] = *reinterpret_cast<const int4*>(a + i * G::YP);
+      if (i < G::W) {
+        w.x += v[i].x;
+        w.y += v[i].y;
+        w.z += v[i].z;
+        w.w += v[i].w;
+      } else {
+        w.x += v[i].x - v[i - G::W].x;
+        w.y += v[i].y - v[i - G::W].y;
+        w.z += v[i].z - v[i - G::W].z;
+        w.w += v[i].w - v[i - G::W].w;
+      }
+      if (i >= G::W - 1) *reinterpret_cast<int4*>(y + (i - G::W + 1) * G::YP) = w;
+    }
+  }
 }
 
 // One output voxel with nearly collinear columns the general way: its limbs
@@ -455,33 +485,9 @@ __global__ void __launch_bounds__(QuadGeom<TY, R>::NT, 1)
     s1[j] = ld_off(slice_s(zb), so + j * 8u * Q.px);
     s2[j] = ld_off(slice_s(zb + 1), so + j * 8u * Q.px);
   }
-  // x window pass from the limb planes to Y: four rows of one limb, a running
-  // sum along the columns
-  auto xpass = [&]() {
-    if (G::XP * G::XJOBS == G::CT || xjob) {
-      int4 v[G::XC + 2 * R];
-      int4 w = make_int4(0, 0, 0, 0);
-#pragma unroll
-      for (int i = 0; i < G::XC + 2 * R; ++i) {
-        v[i] = *reinterpret_cast<const int4*>(xa + i * G::YP);
-        if (i < G::W) {
-          w.x += v[i].x;
-          w.y += v[i].y;
-          w.z += v[i].z;
-          w.w += v[i].w;
-        } else {
-          w.x += v[i].x - v[i - G::W].x;
-          w.y += v[i].y - v[i - G::W].y;
-          w.z += v[i].z - v[i - G::W].z;
-          w.w += v[i].w - v[i - G::W].w;
-        }
-        if (i >= G::W - 1) *reinterpret_cast<int4*>(xy + (i - G::W + 1) * G::YP) = w;
-      }
-    }
-  };
   const int* yv = Y + (size_t)lane * G::YP + row0;
   bar_sync_n<2, G::NT>();  // limbs of slice zb written
-  xpass();
+  quad_xpass<G>(xjob, xa, xy);
   if (zb + 1 < ze) bar_arrive_n<3, G::NT>();  // the limbs may be overwritten
   bar_sync_n<4, G::CT>();                     // the x sums of slice zb are complete
   // what the solve of a slice keeps of its patch sums
@@ -529,31 +535,31 @@ __global__ void __launch_bounds__(QuadGeom<TY, R>::NT, 1)
       int aM[kQuadOut], aG[kQuadOut];
       long long d[kQuadOut];
       km = kg = slow = 0;
-      quad_window<TY, R>(yv, aM);
-      quad_window<TY, R>(yv + G::PY, aG);
-      quad_centred<TY, R>(yv, 6, aM, aM, d);
+      quad_window<G>(yv, aM);
+      quad_window<G>(yv + G::PY, aG);
+      quad_centred<G>(yv, 6, aM, aM, d);
 #pragma unroll
       for (int j = 0; j < kQuadOut; ++j) {
         if (d[j] > P.thr_m) km |= 1u << j;
         im[j] = rsqrt_ftz(ll2f(d[j]));
       }
-      quad_centred<TY, R>(yv, 8, aG, aG, d);
+      quad_centred<G>(yv, 8, aG, aG, d);
 #pragma unroll
       for (int j = 0; j < kQuadOut; ++j) {
         if (d[j] > P.thr_g) kg |= 1u << j;
         ig[j] = rsqrt_ftz(ll2f(d[j]));
       }
-      quad_centred<TY, R>(yv, 10, aM, aG, d);
+      quad_centred<G>(yv, 10, aM, aG, d);
 #pragma unroll
       for (int j = 0; j < kQuadOut; ++j) {
         rmg[j] = ll2f(d[j]) * im[j] * ig[j];
         const float den = 1.0f - rmg[j] * rmg[j];
         if (psg[j] > 0.0f && ((km & kg) >> j & 1) && !(den > 1e-3f)) slow |= 1u << j;
       }
-      quad_centred<TY, R>(yv, 2, sv, aM, d);
+      quad_centred<G>(yv, 2, sv, aM, d);
 #pragma unroll
       for (int j = 0; j < kQuadOut; ++j) fum[j] = ll2f(d[j]);
-      quad_centred<TY, R>(yv, 4, sv, aG, d);
+      quad_centred<G>(yv, 4, sv, aG, d);
 #pragma unroll
       for (int j = 0; j < kQuadOut; ++j) fug[j] = ll2f(d[j]);
       if (slow) {
@@ -577,7 +583,7 @@ __global__ void __launch_bounds__(QuadGeom<TY, R>::NT, 1)
     if (z + 1 < ze) {
       bar_sync_n<4, G::CT>();  // the patch sums of slice z are read
       bar_sync_n<2, G::NT>();  // limbs of slice z+1 written
-      xpass();
+      quad_xpass<G>(xjob, xa, xy);
       if (z + 2 < ze) bar_arrive_n<3, G::NT>();  // the limbs may be overwritten
       bar_sync_n<4, G::CT>();                    // the x sums of slice z+1 are complete
     }

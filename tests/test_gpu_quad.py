@@ -62,3 +62,27 @@ def test_quad_kernel_equals_16_row_kernel(dim, r):
     ctx.set_option(capi.OPTION_TILE_ROWS, 16)
     np.testing.assert_array_equal(ctx.evaluate_batch(mats), got)
     ctx.close()
+
+
+@pytest.mark.parametrize("dim,r", [((32, 24, 12), 4), ((33, 25, 9), 4), ((31, 40, 11), 4),
+                                   ((64, 41, 10), 3), ((37, 23, 7), 3), ((65, 17, 16), 2),
+                                   ((5, 5, 5), 2), ((96, 50, 3), 1), ((1, 64, 33), 1)])
+def test_fixed_quad_kernel_equals_16_row_kernel(dim, r):
+    """HighResolutionModality: Fixed: the structured volume is the static image,
+    the ultrasound (with zeros, which invalidate their patches) is resampled."""
+    case, mats = _case(dim, r)
+    us = case.fixed.copy()
+    us[:, : us.shape[1] // 5] = 0.0
+    fixed = np.ascontiguousarray(case.moving[3:-3, 3:-3, 3:-3])
+    case = synth.Case("3D", case.fixed_geom, fixed, case.fixed_geom, us, [1.0, 1.0, 1.0], r, False,
+                      {}, mats[0])
+    ctx = make_context(case, "f32")
+    ctx.set_option(capi.OPTION_TILE_ROWS, 16)
+    ref = ctx.evaluate_batch(mats)
+    ctx.set_option(capi.OPTION_TILE_ROWS, 0)
+    for zc in (0, 1, 5):
+        ctx.set_option(capi.OPTION_ZCHUNK, zc)
+        np.testing.assert_array_equal(ctx.evaluate_batch(mats), ref)
+    want = oracle_eval(case, mats[0], use_boxsum=False)
+    assert abs(ref[0] - want) <= 1e-5 * abs(want)
+    ctx.close()
