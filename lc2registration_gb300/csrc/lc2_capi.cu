@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/lc2.h"
@@ -1000,16 +1001,21 @@ int launch_mi(lc2_context* c, int cnt) {
     dim3 grid((unsigned)tiles, chunks, n);
     TimerScope ts(c, K_MOMENTS);
     const int st = c->cfg.storage;
-    if (st == LC2_STORE_F16) {
-      lc2::k_mi_range<__half><<<grid, block, 0, c->stream>>>((const __half*)c->d_moving, P, c->d_xf, k0, c->d_rmin, c->d_rmax);
-      lc2::k_mi_hist<__half><<<grid, block, 0, c->stream>>>((const __half*)c->d_moving, P, c->d_xf, k0, c->d_sbin, c->d_rmin, c->d_rmax, c->d_hist);
-    } else if (st == LC2_STORE_BF16) {
-      lc2::k_mi_range<__nv_bfloat16><<<grid, block, 0, c->stream>>>((const __nv_bfloat16*)c->d_moving, P, c->d_xf, k0, c->d_rmin, c->d_rmax);
-      lc2::k_mi_hist<__nv_bfloat16><<<grid, block, 0, c->stream>>>((const __nv_bfloat16*)c->d_moving, P, c->d_xf, k0, c->d_sbin, c->d_rmin, c->d_rmax, c->d_hist);
-    } else {
-      lc2::k_mi_range<float><<<grid, block, 0, c->stream>>>((const float*)c->d_moving, P, c->d_xf, k0, c->d_rmin, c->d_rmax);
-      lc2::k_mi_hist<float><<<grid, block, 0, c->stream>>>((const float*)c->d_moving, P, c->d_xf, k0, c->d_sbin, c->d_rmin, c->d_rmax, c->d_hist);
-    }
+    auto passes = [&](auto* mov) {
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(mov)>>;
+      const bool big = lc2::volume_is_big(P.mx, P.my, P.mz, sizeof(T));
+      auto range = big ? lc2::k_mi_range<T, true> : lc2::k_mi_range<T, false>;
+      auto hist = big ? lc2::k_mi_hist<T, true> : lc2::k_mi_hist<T, false>;
+      range<<<grid, block, 0, c->stream>>>(mov, P, c->d_xf, k0, c->d_rmin, c->d_rmax);
+      hist<<<grid, block, 0, c->stream>>>(mov, P, c->d_xf, k0, c->d_sbin, c->d_rmin, c->d_rmax,
+                                          c->d_hist);
+    };
+    if (st == LC2_STORE_F16)
+      passes((const __half*)c->d_moving);
+    else if (st == LC2_STORE_BF16)
+      passes((const __nv_bfloat16*)c->d_moving);
+    else
+      passes((const float*)c->d_moving);
     lc2::k_mi_part<<<dim3(lc2::kMiParts, n), 256, 0, c->stream>>>(c->d_hist, k0,
                                                                   P.warped_is_high_res, c->d_mipart);
     c->launches += 3;

@@ -174,22 +174,15 @@ __device__ __forceinline__ float fused_sample_inside(const TM* __restrict__ mov,
                                                      const int* sb, const float* sf, int px,
                                                      int py) {
   const float dx = (float)px, dy = (float)py;
-  const float qx = fmaf(A[1], dy, fmaf(A[0], dx, sf[0]));
-  const float qy = fmaf(A[4], dy, fmaf(A[3], dx, sf[1]));
-  const float qz = fmaf(A[7], dy, fmaf(A[6], dx, sf[2]));
-  const float flx = floorf(qx), fly = floorf(qy), flz = floorf(qz);
-  const float rx = qx - flx, ry = qy - fly, rz = qz - flz;
+  unsigned nx, ny, nz;
+  float rx, ry, rz;
+  floor_split(fmaf(A[1], dy, fmaf(A[0], dx, sf[0])), nx, rx);
+  floor_split(fmaf(A[4], dy, fmaf(A[3], dx, sf[1])), ny, ry);
+  floor_split(fmaf(A[7], dy, fmaf(A[6], dx, sf[2])), nz, rz);
   const unsigned mx = (unsigned)P.mx, mxy = (unsigned)P.mx * (unsigned)P.my;
-  const unsigned b = (unsigned)(sb[0] + (int)flx) + (unsigned)(sb[1] + (int)fly) * mx +
-                     (unsigned)(sb[2] + (int)flz) * mxy;
-  float lu0 = ldf(mov, b), lu1 = ldf(mov, b + mxy);
-  float ru0 = ldf(mov, b + 1), ru1 = ldf(mov, b + 1 + mxy);
-  float rb0 = ldf(mov, b + 1 + mx), rb1 = ldf(mov, b + 1 + mx + mxy);
-  float lb0 = ldf(mov, b + mx), lb1 = ldf(mov, b + mx + mxy);
-  float lu = fmaf(rz, lu1 - lu0, lu0), ru = fmaf(rz, ru1 - ru0, ru0);
-  float rb = fmaf(rz, rb1 - rb0, rb0), lb = fmaf(rz, lb1 - lb0, lb0);
-  float l = fmaf(ry, lb - lu, lu), r = fmaf(ry, rb - ru, ru);
-  return fmaf(rx, r - l, l);
+  const unsigned b = ((unsigned)sb[0] - kFloorBias + nx) + ((unsigned)sb[1] - kFloorBias + ny) * mx +
+                     ((unsigned)sb[2] - kFloorBias + nz) * mxy;
+  return trilinear<TM, true>(mov, b, mx, mxy, rx, ry, rz);
 }
 
 // 12 limbs of one point's moment fields: qM, qG, then (lo, hi) of the
@@ -432,7 +425,8 @@ __device__ __forceinline__ bool region_base(const Xform& X, const float* A, cons
       const float lo = fb[a] + fminf(ex, 0.0f) + fminf(e0, e1);
       const float hi = fb[a] + fmaxf(ex, 0.0f) + fmaxf(e0, e1);
       in = in && ((float)ib[a] + lo >= 0.01f) &&
-           ((float)ib[a] + hi <= (float)(dims[a] - 1) - 0.01f);
+           ((float)ib[a] + hi <= (float)(dims[a] - 1) - 0.01f) &&
+           lo > -2097152.0f && hi < 2097152.0f;  // floor_split's range
     }
   }
   return in;
@@ -453,15 +447,15 @@ __device__ __forceinline__ float fused_sample_inside2(const TM* __restrict__ mov
                                                       const int* sb, const float* sf, int px,
                                                       int py) {
   const float dx = (float)px, dy = (float)py;
-  const float qx = fmaf(A[1], dy, fmaf(A[0], dx, sf[0]));
-  const float qy = fmaf(A[4], dy, fmaf(A[3], dx, sf[1]));
-  const float flx = floorf(qx), fly = floorf(qy);
-  const float rx = qx - flx, ry = qy - fly;
+  unsigned nx, ny;
+  float rx, ry;
+  floor_split(fmaf(A[1], dy, fmaf(A[0], dx, sf[0])), nx, rx);
+  floor_split(fmaf(A[4], dy, fmaf(A[3], dx, sf[1])), ny, ry);
   const unsigned mx = (unsigned)P.mx;
-  const unsigned b = (unsigned)(sb[0] + (int)flx) + (unsigned)(sb[1] + (int)fly) * mx;
-  float f0 = ldf(mov, b), f1 = ldf(mov, b + mx);
-  float c0 = ldf(mov, b + 1), c1 = ldf(mov, b + 1 + mx);
-  float xl = fmaf(ry, f1 - f0, f0), xr = fmaf(ry, c1 - c0, c0);
+  const unsigned b = ((unsigned)sb[0] - kFloorBias + nx) + ((unsigned)sb[1] - kFloorBias + ny) * mx;
+  const TM *p0 = mov + (size_t)b, *p1 = mov + (size_t)(b + mx);
+  const float f0 = ldf(p0, 0), f1 = ldf(p1, 0), c0 = ldf(p0, 1), c1 = ldf(p1, 1);
+  const float xl = fmaf(ry, f1 - f0, f0), xr = fmaf(ry, c1 - c0, c0);
   return fmaf(rx, xr - xl, xl);
 }
 
@@ -574,7 +568,7 @@ constexpr int fused_min_blocks(int nd, int ty, int r) {
 // and volume: its strides.
 constexpr int kPreZ = 8;
 
-template <typename TM>
+template <typename TM, bool BIG>
 __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, int mx, int my,
                                                    int mz, int vx, int vy, int vz,
                                                    const Xform* __restrict__ xf, int k0,
@@ -582,8 +576,8 @@ __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, i
                                                    size_t plane, size_t volume) {
   __shared__ int s_ib[kPreZ][3];
   __shared__ float s_fb[kPreZ][3];
-  __shared__ float s_A[9];
-  __shared__ int s_in[kPreZ];
+  __shared__ float4 s_base[kPreZ];
+  __shared__ int s_where[kPreZ];
   const int ntx = (vx + 31) >> 5;
   const int x0 = (blockIdx.x % ntx) * 32, y0 = (blockIdx.x / ntx) * 8;
   const int z0 = blockIdx.y * kPreZ, slot = blockIdx.z;
@@ -592,9 +586,10 @@ __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, i
   if (tid < 3 * kPreZ) {
     const int zs = tid / 3, a = tid - 3 * zs;
     xform_coord(*X, a, x0, y0, z0 + zs, s_ib[zs][a], s_fb[zs][a]);
-  } else if (tid < 3 * kPreZ + 9) {
-    s_A[tid - 3 * kPreZ] = X->ah[tid - 3 * kPreZ];
   }
+  float A[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) A[i] = __ldg(&X->ah[i]);
   __syncthreads();
   if (tid < kPreZ) {
     TileBase T;
@@ -604,27 +599,38 @@ __global__ void __launch_bounds__(256) k_presample(const TM* __restrict__ mov, i
       T.fb[a] = s_fb[tid][a];
     }
 #pragma unroll
-    for (int i = 0; i < 9; ++i) T.A[i] = s_A[i];
-    s_in[tid] = tile_inside(T, mx, my, mz) ? 1 : 0;
+    for (int i = 0; i < 9; ++i) T.A[i] = A[i];
+    s_where[tid] = tile_where(T, mx, my, mz);
+    s_base[tid] = tile_inside_base(T, mx, my);
   }
   __syncthreads();
   const int tx = tid & 31, ty = tid >> 5;
   const int x = x0 + tx, y = y0 + ty;
   if (x >= vx || y >= vy) return;
   float* dst = out + (size_t)slot * volume + (size_t)y * row + x;
+  const float dx = (float)tx, dy = (float)ty;
+  const unsigned umx = (unsigned)mx, mxy = umx * (unsigned)my;
   float v[kPreZ];
 #pragma unroll
   for (int zs = 0; zs < kPreZ; ++zs) {
-    TileBase T;
+    const int where = s_where[zs];
+    if (where == kTileInside) {
+      v[zs] = tile_sample_inside<TM, BIG>(mov, umx, mxy, A, s_base[zs], dx, dy);
+    } else if (where == kTileOutside) {
+      v[zs] = 0.0f;
+    } else if (where == kTileEdge) {
+      v[zs] = tile_sample_edge<TM>(mov, mx, my, mz, s_ib[zs], A, s_fb[zs], dx, dy);
+    } else {
+      TileBase T;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      T.ib[a] = s_ib[zs][a];
-      T.fb[a] = s_fb[zs][a];
+      for (int a = 0; a < 3; ++a) {
+        T.ib[a] = s_ib[zs][a];
+        T.fb[a] = s_fb[zs][a];
+      }
+#pragma unroll
+      for (int i = 0; i < 9; ++i) T.A[i] = A[i];
+      v[zs] = tile_sample<3, TM>(mov, mx, my, mz, T, tx, ty);
     }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) T.A[i] = s_A[i];
-    v[zs] = s_in[zs] ? tile_sample_inside<TM>(mov, mx, my, T, tx, ty)
-                     : tile_sample<3, TM>(mov, mx, my, mz, T, tx, ty);
   }
 #pragma unroll
   for (int zs = 0; zs < kPreZ; ++zs)
@@ -1005,6 +1011,11 @@ cudaError_t fused_launch_grid(const FusedLaunch& L, K kern) {
   return cudaGetLastError();
 }
 
+// Whether a moving volume's byte offsets need more than 32 bits.
+inline bool volume_is_big(int mx, int my, int mz, size_t elem) {
+  return (unsigned long long)mx * my * mz * elem >= 1ull << 32;
+}
+
 // k_presample of transforms [k0, k0 + cnt) into images of these strides.
 template <typename T>
 cudaError_t presample_launch(const void* mov, const FusedParams& P, const Xform* xf, int k0,
@@ -1012,8 +1023,10 @@ cudaError_t presample_launch(const void* mov, const FusedParams& P, const Xform*
                              cudaStream_t stream) {
   const int ntx = (P.vx + 31) / 32, nty = (P.vy + 7) / 8;
   dim3 grid(ntx * nty, (P.vz + kPreZ - 1) / kPreZ, cnt);
-  k_presample<T><<<grid, 256, 0, stream>>>((const T*)mov, P.mx, P.my, P.mz, P.vx, P.vy, P.vz, xf,
-                                           k0, pre, row, plane, volume);
+  auto kern = volume_is_big(P.mx, P.my, P.mz, sizeof(T)) ? k_presample<T, true>
+                                                          : k_presample<T, false>;
+  kern<<<grid, 256, 0, stream>>>((const T*)mov, P.mx, P.my, P.mz, P.vx, P.vy, P.vz, xf, k0, pre,
+                                 row, plane, volume);
   return cudaGetLastError();
 }
 

@@ -222,45 +222,118 @@ __device__ __forceinline__ float tile_sample(const TM* __restrict__ mov, int mx,
   return fmaf(ax.r, xr - xl, xl);
 }
 
-// Whether every sample of a 32 x 8 tile slice from base T lies strictly
-// inside the moving volume (0 <= floor, floor + 1 <= dim - 1 on each axis):
-// the tile's corners bound the affine image, 0.01 voxel covers float rounding.
-__device__ __forceinline__ bool tile_inside(const TileBase& T, int mx, int my, int mz) {
+// Floor and fraction of q, |q| < 2^22, without conversions (FRND and F2I run
+// at a quarter of the rate of additions): q + 1.5 * 2^23 rounded down holds
+// floor(q) in its low mantissa bits; n = floor(q) + kFloorBias.
+constexpr unsigned kFloorBias = 0x4B400000u;
+__device__ __forceinline__ void floor_split(float q, unsigned& n, float& r) {
+  const float m = __fadd_rd(q, 12582912.0f);
+  n = __float_as_uint(m);
+  r = __fsub_rn(q, __fsub_rn(m, 12582912.0f));
+}
+
+// Trilinear sample whose floor corner is voxel b, all eight corners in the
+// volume. BIG: the volume takes 2^32 bytes or more, else the corners are byte
+// offsets from its start.
+template <typename TM, bool BIG>
+__device__ __forceinline__ float trilinear(const TM* __restrict__ mov, unsigned b, unsigned mx,
+                                           unsigned mxy, float rx, float ry, float rz) {
+  const TM *p00, *p01, *p10, *p11;  // rows (y, z): first corner of each
+  if constexpr (BIG) {
+    p00 = mov + (size_t)b;
+    p01 = mov + (size_t)(b + mx);
+    p10 = mov + (size_t)(b + mxy);
+    p11 = mov + (size_t)(b + mx + mxy);
+  } else {
+    const char* base = reinterpret_cast<const char*>(mov);
+    const unsigned o = b * (unsigned)sizeof(TM), oy = mx * (unsigned)sizeof(TM),
+                   oz = mxy * (unsigned)sizeof(TM);
+    p00 = reinterpret_cast<const TM*>(base + o);
+    p01 = reinterpret_cast<const TM*>(base + (o + oy));
+    p10 = reinterpret_cast<const TM*>(base + (o + oz));
+    p11 = reinterpret_cast<const TM*>(base + (o + oy + oz));
+  }
+  const float lu0 = ldf(p00, 0), lu1 = ldf(p10, 0), ru0 = ldf(p00, 1), ru1 = ldf(p10, 1);
+  const float rb0 = ldf(p01, 1), rb1 = ldf(p11, 1), lb0 = ldf(p01, 0), lb1 = ldf(p11, 0);
+  const float lu = fmaf(rz, lu1 - lu0, lu0), ru = fmaf(rz, ru1 - ru0, ru0);
+  const float rb = fmaf(rz, rb1 - rb0, rb0), lb = fmaf(rz, lb1 - lb0, lb0);
+  const float l = fmaf(ry, lb - lu, lu), r = fmaf(ry, rb - ru, ru);
+  return fmaf(rx, r - l, l);
+}
+
+// Where the samples of a 32 x 8 tile slice from base T lie: strictly inside the
+// moving volume (0 <= floor, floor + 1 <= dim - 1 on each axis), all outside
+// along some axis, or neither; kTileAny also where a coordinate may be beyond
+// floor_split's range. The tile's corners bound the affine image, 0.01 voxel
+// covers float rounding.
+enum { kTileAny = 0, kTileInside = 1, kTileOutside = 2, kTileEdge = 3 };
+__device__ __forceinline__ int tile_where(const TileBase& T, int mx, int my, int mz) {
   const int dims[3] = {mx, my, mz};
-  bool in = true;
+  bool in = true, out = false, near = true;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float ex = T.A[3 * a] * 31.0f, ey = T.A[3 * a + 1] * 7.0f;
     const float lo = T.fb[a] + fminf(ex, 0.0f) + fminf(ey, 0.0f);
     const float hi = T.fb[a] + fmaxf(ex, 0.0f) + fmaxf(ey, 0.0f);
-    in = in && ((float)T.ib[a] + lo >= 0.01f) && ((float)T.ib[a] + hi <= (float)(dims[a] - 1) - 0.01f);
+    const float l = (float)T.ib[a] + lo, h = (float)T.ib[a] + hi, end = (float)(dims[a] - 1);
+    in = in && (l >= 0.01f) && (h <= end - 0.01f);
+    out = out || (h < -0.01f - 1e-6f * fabsf(h)) || (l > end + 0.01f + 1e-6f * end);
+    near = near && (lo > -2097152.0f) && (hi < 2097152.0f);
   }
-  return in;
+  return !near ? kTileAny : in ? kTileInside : out ? kTileOutside : kTileEdge;
 }
 
-// tile_sample<3> for a tile slice that tile_inside accepted: no bounds tests,
-// the ceil corner always floor + 1 -- where the fraction is 0 its weight is
-// 0 -- so the value equals tile_sample's bit for bit.
+// Sampling base of a tile slice for kTileInside: fractions, and the base
+// voxel's index minus the biases floor_split adds (modulo 2^32).
+__device__ __forceinline__ float4 tile_inside_base(const TileBase& T, int mx, int my) {
+  const unsigned umx = (unsigned)mx, mxy = umx * (unsigned)my;
+  const unsigned b = (unsigned)T.ib[0] - kFloorBias + ((unsigned)T.ib[1] - kFloorBias) * umx +
+                     ((unsigned)T.ib[2] - kFloorBias) * mxy;
+  return make_float4(T.fb[0], T.fb[1], T.fb[2], __uint_as_float(b));
+}
+
+// tile_sample<3> for a tile slice that is kTileInside: no bounds tests, the
+// ceil corner always floor + 1 -- where the fraction is 0 its weight is 0 --
+// so the value equals tile_sample's bit for bit. A: the transform's steps.
+template <typename TM, bool BIG>
+__device__ __forceinline__ float tile_sample_inside(const TM* __restrict__ mov, unsigned mx,
+                                                    unsigned mxy, const float* A, float4 fb,
+                                                    float dx, float dy) {
+  unsigned nx, ny, nz;
+  float rx, ry, rz;
+  floor_split(fmaf(A[1], dy, fmaf(A[0], dx, fb.x)), nx, rx);
+  floor_split(fmaf(A[4], dy, fmaf(A[3], dx, fb.y)), ny, ry);
+  floor_split(fmaf(A[7], dy, fmaf(A[6], dx, fb.z)), nz, rz);
+  return trilinear<TM, BIG>(mov, __float_as_uint(fb.w) + nx + ny * mx + nz * mxy, mx, mxy, rx, ry, rz);
+}
+
+// tile_sample<3> for a tile slice that is kTileEdge.
 template <typename TM>
-__device__ __forceinline__ float tile_sample_inside(const TM* __restrict__ mov, int mx, int my,
-                                                    const TileBase& T, int tx, int ty) {
-  const float dx = (float)tx, dy = (float)ty;
-  const float qx = fmaf(T.A[1], dy, fmaf(T.A[0], dx, T.fb[0]));
-  const float qy = fmaf(T.A[4], dy, fmaf(T.A[3], dx, T.fb[1]));
-  const float qz = fmaf(T.A[7], dy, fmaf(T.A[6], dx, T.fb[2]));
-  const float flx = floorf(qx), fly = floorf(qy), flz = floorf(qz);
-  const float rx = qx - flx, ry = qy - fly, rz = qz - flz;
-  const unsigned umx = (unsigned)mx, mxy = (unsigned)mx * (unsigned)my;
-  const unsigned b = (unsigned)(T.ib[0] + (int)flx) + (unsigned)(T.ib[1] + (int)fly) * umx +
-                     (unsigned)(T.ib[2] + (int)flz) * mxy;
-  float lu0 = ldf(mov, b), lu1 = ldf(mov, b + mxy);
-  float ru0 = ldf(mov, b + 1), ru1 = ldf(mov, b + 1 + mxy);
-  float rb0 = ldf(mov, b + 1 + umx), rb1 = ldf(mov, b + 1 + umx + mxy);
-  float lb0 = ldf(mov, b + umx), lb1 = ldf(mov, b + umx + mxy);
-  float lu = fmaf(rz, lu1 - lu0, lu0), ru = fmaf(rz, ru1 - ru0, ru0);
-  float rb = fmaf(rz, rb1 - rb0, rb0), lb = fmaf(rz, lb1 - lb0, lb0);
-  float l = fmaf(ry, lb - lu, lu), r = fmaf(ry, rb - ru, ru);
-  return fmaf(rx, r - l, l);
+__device__ __forceinline__ float tile_sample_edge(const TM* __restrict__ mov, int mx, int my, int mz,
+                                                  const int* ib, const float* A, const float* fb,
+                                                  float dx, float dy) {
+  unsigned n[3];
+  float r[3];
+  int f[3], c[3];
+  const int dims[3] = {mx, my, mz};
+  bool ok = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    floor_split(fmaf(A[3 * a + 1], dy, fmaf(A[3 * a], dx, fb[a])), n[a], r[a]);
+    f[a] = ib[a] + (int)(n[a] - kFloorBias);
+    c[a] = r[a] > 0.0f ? 1 : 0;  // ceil corner = floor where the fraction is 0
+    ok = ok && f[a] >= 0 && f[a] + c[a] <= dims[a] - 1;
+  }
+  if (!ok) return 0.0f;
+  const unsigned umx = (unsigned)mx, mxy = umx * (unsigned)my;
+  const TM* p = mov + ((size_t)(unsigned)f[0] + (size_t)(unsigned)f[1] * umx + (size_t)(unsigned)f[2] * mxy);
+  const size_t ox = c[0], oy = c[1] ? umx : 0, oz = c[2] ? mxy : 0;
+  const float lu0 = ldf(p, 0), lu1 = ldf(p, oz), ru0 = ldf(p, ox), ru1 = ldf(p, ox + oz);
+  const float rb0 = ldf(p, ox + oy), rb1 = ldf(p, ox + oy + oz), lb0 = ldf(p, oy), lb1 = ldf(p, oy + oz);
+  const float lu = fmaf(r[2], lu1 - lu0, lu0), ru = fmaf(r[2], ru1 - ru0, ru0);
+  const float rb = fmaf(r[2], rb1 - rb0, rb0), lb = fmaf(r[2], lb1 - lb0, lb0);
+  const float l = fmaf(r[1], lb - lu, lu), rr = fmaf(r[1], rb - ru, ru);
+  return fmaf(r[0], rr - l, l);
 }
 
 // One CTA = 32x8 virtual voxels of one z-slice of one transform slot.

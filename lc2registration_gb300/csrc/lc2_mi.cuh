@@ -60,45 +60,75 @@ constexpr int kMiChunk = 64;  // most slices per range / histogram CTA
 constexpr int kMiParts = 32;  // entropy CTAs per transform (8 warped bins each)
 
 // Sampling bases of a CTA's tile for its slices [zb, ze), one per thread, in
-// shared memory, and whether each slice samples strictly inside the warped
-// image (tile_inside); the caller synchronises.
+// shared memory, and where each slice samples (tile_where); the caller
+// synchronises.
+struct MiBases {
+  int ib[kMiChunk][3];
+  float fb[kMiChunk][3];
+  float4 base[kMiChunk];
+  int where[kMiChunk];
+};
 __device__ __forceinline__ void mi_bases(const Xform* X, const MiParams& P, int x0, int y0,
-                                         int zb, int ze, TileBase* T, int* inside) {
+                                         int zb, int ze, MiBases& B) {
   const int t = threadIdx.y * blockDim.x + threadIdx.x;
   if (zb + t < ze) {
-    tile_base(X, x0, y0, zb + t, T[t]);
-    inside[t] = tile_inside(T[t], P.mx, P.my, P.mz) ? 1 : 0;
+    TileBase T;
+    tile_base(X, x0, y0, zb + t, T);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      B.ib[t][a] = T.ib[a];
+      B.fb[t][a] = T.fb[a];
+    }
+    B.base[t] = tile_inside_base(T, P.mx, P.my);
+    B.where[t] = tile_where(T, P.mx, P.my, P.mz);
   }
 }
 
-template <typename TM>
+template <typename TM, bool BIG>
 __device__ __forceinline__ float mi_sample(const TM* __restrict__ mov, const MiParams& P,
-                                           const TileBase& T, int inside) {
-  return inside ? tile_sample_inside<TM>(mov, P.mx, P.my, T, threadIdx.x, threadIdx.y)
-                : tile_sample<3, TM>(mov, P.mx, P.my, P.mz, T, threadIdx.x, threadIdx.y);
+                                           const float* A, const MiBases& B, int t) {
+  const int where = B.where[t];
+  const float dx = (float)threadIdx.x, dy = (float)threadIdx.y;
+  if (where == kTileInside)
+    return tile_sample_inside<TM, BIG>(mov, (unsigned)P.mx, (unsigned)P.mx * (unsigned)P.my, A,
+                                       B.base[t], dx, dy);
+  if (where == kTileOutside) return 0.0f;
+  if (where == kTileEdge)
+    return tile_sample_edge<TM>(mov, P.mx, P.my, P.mz, B.ib[t], A, B.fb[t], dx, dy);
+  TileBase T;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    T.ib[a] = B.ib[t][a];
+    T.fb[a] = B.fb[t][a];
+  }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) T.A[i] = A[i];
+  return tile_sample<3, TM>(mov, P.mx, P.my, P.mz, T, threadIdx.x, threadIdx.y);
 }
 
 // Range of the warped image of each transform. Grid (tiles of 32 x 8, z
 // chunks, transforms), block (32, 8).
-template <typename TM>
+template <typename TM, bool BIG>
 __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, MiParams P,
                                                   const Xform* __restrict__ xf, int k0,
                                                   unsigned* __restrict__ rmin,
                                                   unsigned* __restrict__ rmax) {
-  __shared__ TileBase T[kMiChunk];
-  __shared__ int inside[kMiChunk];
+  __shared__ MiBases B;
   __shared__ float red[2][8];
   const int ntx = (P.vx + 31) / 32;
   const int x0 = (blockIdx.x % ntx) * 32, y0 = (blockIdx.x / ntx) * 8;
   const int zb = blockIdx.y * P.zchunk, ze = min(zb + P.zchunk, P.vz);
   const int slot = blockIdx.z;
-  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, T, inside);
+  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, B);
+  float A[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) A[i] = __ldg(&xf[k0 + slot].ah[i]);
   __syncthreads();
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
   float lo = INFINITY, hi = -INFINITY;
   if (x < P.vx && y < P.vy) {
     for (int z = zb; z < ze; ++z) {
-      const float v = mi_sample<TM>(mov, P, T[z - zb], inside[z - zb]);
+      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb);
       lo = fminf(lo, v);
       hi = fmaxf(hi, v);
     }
@@ -153,15 +183,14 @@ __device__ __forceinline__ void mi_table_add(int* tkey, unsigned* tcnt, unsigned
 // the warped image's bins in its range. Grid and block as k_mi_range. With
 // P.table a CTA first merges its counts in a shared table (neighbouring
 // voxels share bins), then adds each key once.
-template <typename TM>
+template <typename TM, bool BIG>
 __global__ void __launch_bounds__(256) k_mi_hist(const TM* __restrict__ mov, MiParams P,
                                                  const Xform* __restrict__ xf, int k0,
                                                  const unsigned char* __restrict__ sbin,
                                                  const unsigned* __restrict__ rmin,
                                                  const unsigned* __restrict__ rmax,
                                                  unsigned* __restrict__ hist) {
-  __shared__ TileBase T[kMiChunk];
-  __shared__ int inside[kMiChunk];
+  __shared__ MiBases B;
   __shared__ int tkey[kMiTable];
   __shared__ unsigned tcnt[kMiTable];
   const int ntx = (P.vx + 31) / 32;
@@ -176,7 +205,10 @@ __global__ void __launch_bounds__(256) k_mi_hist(const TM* __restrict__ mov, MiP
       tcnt[i] = 0;
     }
   }
-  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, T, inside);
+  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, B);
+  float A[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) A[i] = __ldg(&xf[k0 + slot].ah[i]);
   __syncthreads();
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
   const bool in = x < P.vx && y < P.vy;
@@ -187,7 +219,7 @@ __global__ void __launch_bounds__(256) k_mi_hist(const TM* __restrict__ mov, MiP
   for (int z = zb; z < ze; ++z) {
     int key = -1;
     if (in) {
-      const float v = mi_sample<TM>(mov, P, T[z - zb], inside[z - zb]);
+      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb);
       const int wb = mi_bin(v, lo, sc);
       const int sb = sbin[((size_t)z * P.vy + y) * P.vx + x];
       if (wb >= 0 && wb < kMiBins)
