@@ -873,6 +873,13 @@ __global__ void __launch_bounds__(kNT) k_moments(const TU* __restrict__ Ubase,
   flush_sums(acc_m, acc_s, acc + 2 * (size_t)(k0 + slot));
 }
 
+// Raises a flag in pinned host memory after everything the block wrote there.
+__device__ __forceinline__ void raise_flag(unsigned* flag) {
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned*>(flag) = 1u;
+}
+
 // float -> storage type conversion of a device buffer
 template <typename T>
 __global__ void k_convert(const float* __restrict__ in, T* __restrict__ out, size_t n) {

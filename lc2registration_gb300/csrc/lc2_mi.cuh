@@ -246,14 +246,15 @@ __global__ void __launch_bounds__(256) k_mi_hist(const TM* __restrict__ mov, MiP
 // or its columns (key = warped + 256 static). part[k][b] = (sum over its
 // joint bins of c ln c, sum over its warped marginals of c ln c). Grid
 // (kMiParts, transforms), 256 threads.
-__global__ void __launch_bounds__(256) k_mi_part(const unsigned* __restrict__ hist, int k0,
+// The histogram is left zeroed for the next batch.
+__global__ void __launch_bounds__(256) k_mi_part(unsigned* __restrict__ hist, int k0,
                                                  int warped_is_high_res,
                                                  double* __restrict__ part) {
   constexpr int WB = kMiBins / kMiParts;  // warped bins per part
   __shared__ unsigned marg[WB];
   __shared__ double red[2][8];
   const int k = k0 + blockIdx.y, b = blockIdx.x, tid = threadIdx.x;
-  const unsigned* h = hist + (size_t)k * kMiHist;
+  unsigned* h = hist + (size_t)k * kMiHist;
   if (tid < WB) marg[tid] = 0;
   __syncthreads();
   double sj = 0.0;
@@ -264,8 +265,10 @@ __global__ void __launch_bounds__(256) k_mi_part(const unsigned* __restrict__ hi
     const int wl = warped_is_high_res ? j : (tid & (WB - 1));
     const int sbn = warped_is_high_res ? tid : (tid >> 3) + 32 * j;
     const int w = WB * b + wl;
-    const unsigned c = warped_is_high_res ? h[sbn + kMiBins * w] : h[w + kMiBins * sbn];
+    unsigned* hc = warped_is_high_res ? h + (sbn + kMiBins * w) : h + (w + kMiBins * sbn);
+    const unsigned c = *hc;
     if (c) {
+      *hc = 0;
       sj += (double)c * log((double)c);
       atomicAdd(&marg[wl], c);
     }
@@ -285,22 +288,28 @@ __global__ void __launch_bounds__(256) k_mi_part(const unsigned* __restrict__ hi
 }
 
 // NMI of each transform from its parts, summed in part order.
-// h_static: entropy of the static image; voxels: virtual-grid size.
+// h_static: entropy of the static image; voxels: virtual-grid size. The ranges
+// are reset for the next batch; flag as in k_finalize.
 __global__ void k_mi_nmi(const double* __restrict__ part, int cnt, double h_static,
-                         double voxels, double* __restrict__ out) {
+                         double voxels, unsigned* __restrict__ rmin, unsigned* __restrict__ rmax,
+                         double* __restrict__ out, unsigned* __restrict__ flag) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= cnt) return;
-  double a = 0.0, b = 0.0;
-  for (int i = 0; i < kMiParts; ++i) {
-    a += part[((size_t)k * kMiParts + i) * 2];
-    b += part[((size_t)k * kMiParts + i) * 2 + 1];
+  if (k < cnt) {
+    double a = 0.0, b = 0.0;
+    for (int i = 0; i < kMiParts; ++i) {
+      a += part[((size_t)k * kMiParts + i) * 2];
+      b += part[((size_t)k * kMiParts + i) * 2 + 1];
+    }
+    const double ln_n = log(voxels);
+    const double hj = ln_n - a / voxels;  // H(U, M)
+    const double hw = ln_n - b / voxels;  // H(warped)
+    double v = (h_static + hw) / hj;
+    if (isnan(v) || isinf(v)) v = 0.0;
+    rmin[k] = 0xffffffffu;
+    rmax[k] = 0u;
+    out[k] = v;
   }
-  const double ln_n = log(voxels);
-  const double hj = ln_n - a / voxels;  // H(U, M)
-  const double hw = ln_n - b / voxels;  // H(warped)
-  double v = (h_static + hw) / hj;
-  if (isnan(v) || isinf(v)) v = 0.0;
-  out[k] = v;
+  if (flag) raise_flag(flag);
 }
 
 }  // namespace lc2
