@@ -265,32 +265,105 @@ struct lc2_context {
 };
 
 namespace lc2 {
-// Exact window sum of width 2r+1 along one axis (0 = x, 1 = y, 2 = z) with
-// zero padding; one thread per line of the (nx, ny, nz) grid.
+// Exact window sums of width 2r+1 with zero padding (r <= 12). Bound by their
+// one read and one write of the image. Along x: a warp per row, its values
+// staged in shared memory 128 at a time, each lane summing the windows of four
+// interleaved columns (a running sum per lane would read with a stride).
 template <typename T>
-__global__ void k_box_line(const T* __restrict__ in, T* __restrict__ out, int nx, int ny,
-                           int nz, int axis, int r) {
-  const long long line = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t base, stride;
-  int len;
-  if (axis == 0) {
-    if (line >= (long long)ny * nz) return;
-    base = (size_t)line * nx; stride = 1; len = nx;
-  } else if (axis == 1) {
-    if (line >= (long long)nx * nz) return;
-    base = (size_t)(line / nx) * nx * ny + (size_t)(line % nx); stride = nx; len = ny;
-  } else {
-    if (line >= (long long)nx * ny) return;
-    base = (size_t)line; stride = (size_t)nx * ny; len = nz;
+__global__ void __launch_bounds__(256) k_box_x(const T* __restrict__ in, T* __restrict__ out,
+                                               int nx, long long rows, int r) {
+  __shared__ T s_v[8][128 + 24];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long row = (long long)blockIdx.x * 8 + w;
+  if (row >= rows) return;
+  const T* src = in + row * nx;
+  T* dst = out + row * nx;
+  T* v = s_v[w];
+  for (int x0 = 0; x0 < nx; x0 += 128) {
+    __syncwarp();
+    for (int i = lane; i < 128 + 2 * r; i += 32) {
+      const int x = x0 - r + i;
+      v[i] = (x >= 0 && x < nx) ? src[x] : T(0);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = lane + 32 * k;
+      if (x0 + i < nx) {
+        T a = 0;
+        for (int j = 0; j <= 2 * r; ++j) a += v[i + j];
+        dst[x0 + i] = a;
+      }
+    }
   }
+}
+
+// Along y or z: a thread per segment of kBoxSeg outputs of a line, a running
+// sum; neighbouring threads take neighbouring lines. Lines are `inner`
+// consecutive elements apart by `stride`, `outer` groups `group` apart.
+constexpr int kBoxSeg = 16;
+template <typename T>
+__global__ void __launch_bounds__(256) k_box_line(const T* __restrict__ in, T* __restrict__ out,
+                                                  long long inner, long long outer, size_t stride,
+                                                  size_t group, int len, int r) {
+  const long long line = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (line >= inner * outer) return;
+  const long long g = line / inner;
+  const size_t base = (size_t)g * group + (size_t)(line - g * inner);
+  const int j0 = blockIdx.y * kBoxSeg, j1 = min(j0 + kBoxSeg, len);
   T a = 0;
-  for (int i = 0; i <= r && i < len; ++i) a += in[base + i * stride];
-  out[base] = a;
-  for (int i = 1; i < len; ++i) {
-    if (i + r < len) a += in[base + (size_t)(i + r) * stride];
-    if (i - r - 1 >= 0) a -= in[base + (size_t)(i - r - 1) * stride];
-    out[base + (size_t)i * stride] = a;
+  for (int j = max(j0 - r, 0); j < min(j0 + r, len); ++j) a += in[base + (size_t)j * stride];
+#pragma unroll 4
+  for (int j = j0; j < j1; ++j) {
+    if (j + r < len) a += in[base + (size_t)(j + r) * stride];
+    out[base + (size_t)j * stride] = a;
+    if (j - r >= 0) a -= in[base + (size_t)(j - r) * stride];
   }
+}
+
+// Static ultrasound: quantised values, and their squares with a mark at bit
+// kInvalidBit for a value <= 1e-6 (cu_lc2_3d.cu:223-243); a window's marks add
+// up above its sum of squares (< 2^50).
+constexpr int kInvalidBit = 52;
+template <typename TU>
+__global__ void k_static_u(const TU* __restrict__ U, size_t n, float qu, int* __restrict__ q,
+                           long long* __restrict__ w) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const float u = ldf(U, i);
+    const int v = quant(u, qu);
+    q[i] = v;
+    w[i] = (long long)v * v + (u > 1e-6f ? 0ll : 1ll << kInvalidBit);
+  }
+}
+
+// Weighting factor of every voxel from the window sums S_U and w, as
+// solve_centred computes it (0 where the window leaves the grid, holds an
+// invalid value or has no variance), and the exact sum of all of them.
+__global__ void __launch_bounds__(256) k_sigma(const int* __restrict__ su,
+                                               const long long* __restrict__ w, int nx, int ny,
+                                               int nz, int r, int rz, long long n,
+                                               long long thr_var, float sig_scale, float sum_scale,
+                                               float* __restrict__ sigma,
+                                               unsigned long long* __restrict__ sum) {
+  const size_t nv = (size_t)nx * ny * nz;
+  long long acc = 0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t l = i / nx;
+    const int x = (int)(i - l * nx), z = (int)(l / ny), y = (int)(l - (size_t)z * ny);
+    float sg = 0.0f;
+    const long long s = su[i], uu = w[i];
+    if (x >= r && x + r < nx && y >= r && y + r < ny && z >= rz && z + rz < nz &&
+        (uu >> kInvalidBit) == 0) {
+      const long long d = n * uu - s * s;
+      if (d > thr_var) sg = sqrtf(ll2f(d)) * sig_scale;
+    }
+    sigma[i] = sg;
+    acc += __float2int_rn(sg * sum_scale);
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(sum, (unsigned long long)acc);
 }
 
 // An image of rows nx and ny rows per slice into padded strides.
@@ -303,18 +376,14 @@ __global__ void k_pad(const int* __restrict__ in, int nx, int ny, size_t n, int*
   }
 }
 
-// The static ultrasound's fields in padded strides: quantised values, and
-// (weighting factor bits, window sum) pairs.
-template <typename TU>
-__global__ void k_pad_static(const TU* __restrict__ U, float qu, const float* __restrict__ sig,
-                             const int* __restrict__ su, int nx, int ny, size_t n,
-                             int* __restrict__ uq, int2* __restrict__ ss, int row, size_t plane) {
+// (weighting factor bits, window sum) pairs of the static ultrasound in padded
+// strides.
+__global__ void k_pad_static(const float* __restrict__ sig, const int* __restrict__ su, int nx,
+                             int ny, size_t n, int2* __restrict__ ss, int row, size_t plane) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const size_t l = i / nx, z = l / ny;
-    const size_t o = z * plane + (l - z * ny) * row + (i - l * nx);
-    uq[o] = quant(ldf(U, i), qu);
-    ss[o] = make_int2(__float_as_int(sig[i]), su[i]);
+    ss[z * plane + (l - z * ny) * row + (i - l * nx)] = make_int2(__float_as_int(sig[i]), su[i]);
   }
 }
 
@@ -1206,9 +1275,10 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
   // padded static fields: quantised ultrasound and its (sigma, S_U), or M and G
   if (c->quad) h += (hrm ? sizeof(int) + sizeof(int2) : 2 * sizeof(int)) * c->lay.volume();
   *held = h;
-  *peak_extra = std::max(c->nm, c->nf) * sizeof(float);
-  if (!hrm && !c->mi)  // temporaries of the static sums
-    *peak_extra = std::max(*peak_extra, c->nv * (sizeof(int) + sizeof(long long)));
+  // both images, and the temporaries of the static sums
+  *peak_extra = (c->nm + c->nf) * sizeof(float);
+  if (!c->mi)
+    *peak_extra += c->nv * (hrm ? 2 * sizeof(long long) : 2 * sizeof(int) + sizeof(long long));
 }
 
 int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
@@ -1497,14 +1567,24 @@ int image_absmax(const float* img, size_t n, const char* what, float* out) {
 // Largest |value| of a device float image (as float bits, atomicMax on the
 // non-negative bit patterns orders them like the values) and a flag for
 // NaN/Inf anywhere in it. out[0] and out[1] must start at zero.
-__global__ void k_absmax_flag(const float* __restrict__ a, size_t n, unsigned int* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_absmax_flag(const float* __restrict__ a, size_t n,
+                                                     unsigned int* __restrict__ out) {
   unsigned int m = 0, bad = 0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const float v = a[i];
+  auto take = [&](float v) {
     if (!isfinite(v)) bad = 1;
     m = max(m, __float_as_uint(fabsf(v)));
+  };
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  const size_t n4 = (reinterpret_cast<uintptr_t>(a) & 15) == 0 ? n / 4 : 0;
+#pragma unroll 4
+  for (size_t i = t; i < n4; i += step) {
+    const float4 v = reinterpret_cast<const float4*>(a)[i];
+    take(v.x);
+    take(v.y);
+    take(v.z);
+    take(v.w);
   }
+  for (size_t i = 4 * n4 + t; i < n; i += step) take(a[i]);
   for (int o = 16; o > 0; o >>= 1) {
     m = max(m, __shfl_down_sync(0xffffffffu, m, o));
     bad |= __shfl_down_sync(0xffffffffu, bad, o);
@@ -1515,99 +1595,133 @@ __global__ void k_absmax_flag(const float* __restrict__ a, size_t n, unsigned in
   }
 }
 
-// Host float image -> device buffer of the storage type (synchronous). A
-// device-resident source (lc2_set_images_device) is converted in place of
-// the staging copy.
-int upload_image(lc2_context* c, const float* host, size_t n, void* dst, int storage,
-                 bool on_device = false) {
-  if (on_device) {
-    LC2_TRY(convert_to_storage(c, host, dst, n, storage));
-    LC2_CUDA(cudaStreamSynchronize(c->stream));
-    return LC2_OK;
-  }
-  float* tmp = nullptr;
-  LC2_CUDA(dev_alloc((void**)&tmp, sizeof(float) * n, c->stream));
-  struct Free {
-    float* p;
-    cudaStream_t st;
-    ~Free() { dev_free(p, st); }
-  } guard{tmp, c->stream};
-  LC2_CUDA(cudaMemcpyAsync(tmp, host, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
-  LC2_TRY(convert_to_storage(c, tmp, dst, n, storage));
+// Largest |value| of n device floats; *bad: NaN/Inf among them. For two images.
+int device_absmax(lc2_context* c, const float* a, size_t na, const float* b, size_t nb, float mx[2],
+                  bool bad[2]) {
+  unsigned int* flags = reinterpret_cast<unsigned int*>(c->d_acc);  // 4 words, reset below
+  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
+  const int blocks = 152 * 6;
+  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(a, na, flags);
+  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(b, nb, flags + 2);
+  LC2_CUDA(cudaGetLastError());
+  unsigned int h[4] = {0, 0, 0, 0};
+  LC2_CUDA(cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
   LC2_CUDA(cudaStreamSynchronize(c->stream));
+  for (int i = 0; i < 2; ++i) {
+    std::memcpy(&mx[i], &h[2 * i], 4);
+    bad[i] = h[2 * i + 1] != 0;
+  }
   return LC2_OK;
 }
 
-// Everything that depends on the fixed image, given the moving image's
-// largest |value| (its scale enters the fixed-point parameters): the fixed
-// image on the virtual grid, the fixed-point parameters and, for a static
-// ultrasound, the weighting factors and their sum.
-// Window sums of the quantised static ultrasound per voxel (the S_U of the
-// fused kernels), by exact separable passes through scratch slot 0.
-int static_window_sum(lc2_context* c) {
+// A temporary device buffer, freed in stream order at the end of its scope.
+template <typename T>
+struct TempBuffer {
+  T* p = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t alloc(size_t n, cudaStream_t s) {
+    st = s;
+    return dev_alloc((void**)&p, n * sizeof(T), s);
+  }
+  ~TempBuffer() { dev_free(p, st); }
+};
+
+// Window sums over the context's patch of the image in a, into out or, without
+// one, into b (3D) or a (2D); returns where. a and b are overwritten; a pass
+// never writes what it reads.
+template <typename T>
+T* box_sums(lc2_context* c, T* a, T* b, T* out = nullptr) {
+  const long long nx = c->virt.dim[0], ny = c->virt.dim[1], nz = c->virt.dim[2];
+  const int r = c->cfg.patch_size;
+  auto line = [&](const T* src, T* dst, long long inner, long long outer, size_t stride, size_t group,
+                  long long len) {
+    dim3 grid((unsigned)((inner * outer + 255) / 256),
+              (unsigned)((len + lc2::kBoxSeg - 1) / lc2::kBoxSeg));
+    lc2::k_box_line<T><<<grid, 256, 0, c->stream>>>(src, dst, inner, outer, stride, group, (int)len, r);
+    ++c->launches;
+  };
+  lc2::k_box_x<T><<<(unsigned)((ny * nz + 7) / 8), 256, 0, c->stream>>>(a, b, (int)nx, ny * nz, r);
+  ++c->launches;
+  if (c->lc2_nd == 2) {
+    if (!out) out = a;
+    line(b, out, nx, nz, (size_t)nx, (size_t)(nx * ny), ny);
+    return out;
+  }
+  line(b, a, nx, nz, (size_t)nx, (size_t)(nx * ny), ny);
+  if (!out) out = b;
+  line(a, out, nx * ny, 1, (size_t)(nx * ny), 0, nz);
+  return out;
+}
+
+// Static ultrasound: its window sums S_U, weighting factors and their sum, by
+// exact box sums. With it, the checks on the device and the fixed image through
+// k_presample, lc2_set_images takes 24.5 -> 1.6 ms on 256^3 host volumes and
+// 2.3 -> 0.29 ms for 128^3 -> 96^3 (the generic moments kernel alone took 1.4,
+// line-by-line sums 0.4 and the host's scan for NaN about 20 ms).
+int static_sums(lc2_context* c) {
   const lc2_geometry& v = c->virt;
   const size_t nv = c->nv;
-  int* ta = reinterpret_cast<int*>(c->d_scratch);
-  int* tb = ta + nv;  // the slot holds two planes of nv floats
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
   const int st = c->cfg.storage;
-  if (st == LC2_STORE_F16)
-    lc2::k_quant_static<__half><<<blocks, 256, 0, c->stream>>>((const __half*)c->d_static, nv, c->fp.qu, ta);
-  else if (st == LC2_STORE_BF16)
-    lc2::k_quant_static<__nv_bfloat16><<<blocks, 256, 0, c->stream>>>((const __nv_bfloat16*)c->d_static, nv, c->fp.qu, ta);
-  else
-    lc2::k_quant_static<float><<<blocks, 256, 0, c->stream>>>((const float*)c->d_static, nv, c->fp.qu, ta);
   const int nx = v.dim[0], ny = v.dim[1], nz = v.dim[2], r = c->cfg.patch_size;
-  auto pass = [&](const int* in, int* out, int axis, long long lines) {
-    lc2::k_box_line<int><<<(unsigned)((lines + 127) / 128), 128, 0, c->stream>>>(in, out, nx, ny, nz,
-                                                                            axis, r);
+  int* q = reinterpret_cast<int*>(c->d_scratch);
+  int* tq = q + nv;  // the slot holds two planes of nv floats
+  TempBuffer<long long> w, tw;
+  LC2_CUDA(w.alloc(nv, c->stream));
+  LC2_CUDA(tw.alloc(nv, c->stream));
+  auto with_u = [&](auto* u) {
+    lc2::k_static_u<<<blocks, 256, 0, c->stream>>>(u, nv, c->fp.qu, q, w.p);
   };
-  pass(ta, tb, 0, (long long)ny * nz);
-  if (c->lc2_nd == 3) {
-    pass(tb, ta, 1, (long long)nx * nz);
-    pass(ta, c->d_su, 2, (long long)nx * ny);
-  } else {
-    pass(tb, c->d_su, 1, (long long)nx * nz);
-  }
-  c->launches += (c->lc2_nd == 3) ? 4 : 3;
+  if (st == LC2_STORE_F16)
+    with_u((const __half*)c->d_static);
+  else if (st == LC2_STORE_BF16)
+    with_u((const __nv_bfloat16*)c->d_static);
+  else
+    with_u((const float*)c->d_static);
+  ++c->launches;
   if (c->quad) {
-    const size_t at = c->lay.first() + c->lay.origin();
     LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.volume() * sizeof(int), c->stream));
     LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.volume() * sizeof(int2), c->stream));
-    auto pad = [&](auto* u) {
-      lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(u, c->fp.qu, c->d_sigma, c->d_su, nx, ny, nv,
-                                                       c->d_uq + at, c->d_ss + at, c->lay.px,
-                                                       c->lay.slice());
-    };
-    if (st == LC2_STORE_F16)
-      pad((const __half*)c->d_static);
-    else if (st == LC2_STORE_BF16)
-      pad((const __nv_bfloat16*)c->d_static);
-    else
-      pad((const float*)c->d_static);
+    lc2::k_pad<<<blocks, 256, 0, c->stream>>>(q, nx, ny, nv,
+                                              c->d_uq + c->lay.first() + c->lay.origin(), c->lay.px,
+                                              c->lay.slice());
+    ++c->launches;
+  }
+  box_sums(c, q, tq, c->d_su);
+  const long long* sums = box_sums(c, w.p, tw.p);
+  c->acc_clean = false;
+  LC2_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long), c->stream));
+  lc2::k_sigma<<<blocks, 256, 0, c->stream>>>(c->d_su, sums, nx, ny, nz, r, c->lc2_nd == 3 ? r : 0,
+                                              (long long)c->n, c->mp.thr_var, c->mp.sig_scale,
+                                              c->mp.sum_scale, c->d_sigma, c->d_acc);
+  ++c->launches;
+  if (c->quad) {
+    lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(
+        c->d_sigma, c->d_su, nx, ny, nv, c->d_ss + c->lay.first() + c->lay.origin(), c->lay.px,
+        c->lay.slice());
     ++c->launches;
   }
   LC2_CUDA(cudaGetLastError());
+  unsigned long long sum = 0;
+  LC2_CUDA(cudaMemcpyAsync(&sum, c->d_acc, sizeof(sum), cudaMemcpyDeviceToHost, c->stream));
   LC2_CUDA(cudaStreamSynchronize(c->stream));
+  c->sigma_sum = (long long)sum;
   return LC2_OK;
 }
 
 // Resampled ultrasound: quantised static image and Sobel, their exact window
-// sums and centred sums, once per context (the fields k_fused_fixed* read).
+// sums and centred sums, once per context (the fields k_fixed_quad and
+// k_fused_fixed* read).
 int fixed_static_sums(lc2_context* c) {
   const lc2_geometry& v = c->virt;
   const size_t nv = c->nv;
-  const int nx = v.dim[0], ny = v.dim[1], nz = v.dim[2], r = c->cfg.patch_size;
-  int* ti = nullptr;
-  long long* tl = nullptr;
-  LC2_CUDA(dev_alloc((void**)&ti, nv * sizeof(int), c->stream));
-  struct Free {
-    void* p;
-    cudaStream_t st;
-    ~Free() { dev_free(p, st); }
-  } g1{ti, c->stream};
-  LC2_CUDA(dev_alloc((void**)&tl, nv * sizeof(long long), c->stream));
-  Free g2{tl, c->stream};
+  const int nx = v.dim[0], ny = v.dim[1];
+  TempBuffer<int> ti, tj;
+  TempBuffer<long long> tl;
+  LC2_CUDA(ti.alloc(nv, c->stream));
+  LC2_CUDA(tj.alloc(nv, c->stream));
+  LC2_CUDA(tl.alloc(nv, c->stream));
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
   lc2::k_fixed_quant<<<blocks, 256, 0, c->stream>>>((const float*)c->d_static, c->d_gstatic, nv,
                                                     c->fp.qm, c->fp.qg, c->d_fq, c->d_fd);
@@ -1620,43 +1734,24 @@ int fixed_static_sums(lc2_context* c) {
           c->lay.slice());
     c->launches += 2;
   }
-  auto pass = [&](auto* in, auto* out, int axis) {
-    const long long lines = axis == 0 ? (long long)ny * nz : axis == 1 ? (long long)nx * nz
-                                                                       : (long long)nx * ny;
-    lc2::k_box_line<<<(unsigned)((lines + 127) / 128), 128, 0, c->stream>>>(in, out, nx, ny, nz,
-                                                                            axis, r);
-    ++c->launches;
-  };
-  // S_M, S_G: q -> s through x, y (, z) passes
+  // S_M, S_G (from a copy of q, which stays), then S_MM, S_GG, S_MG in place in d
   for (int f = 0; f < 2; ++f) {
-    int* q = c->d_fq + f * nv;
-    int* o = c->d_fs + f * nv;
-    if (c->lc2_nd == 3) {
-      pass(q, o, 0);
-      pass(o, ti, 1);
-      pass(ti, o, 2);
-    } else {
-      pass(q, ti, 0);
-      pass(ti, o, 1);
-    }
+    LC2_CUDA(cudaMemcpyAsync(ti.p, c->d_fq + f * nv, nv * sizeof(int), cudaMemcpyDeviceToDevice,
+                             c->stream));
+    box_sums(c, ti.p, tj.p, c->d_fs + f * nv);
   }
-  // S_MM, S_GG, S_MG in place in d
   for (int f = 0; f < 3; ++f) {
-    long long* p = c->d_fd + f * nv;
-    pass(p, tl, 0);
-    pass(tl, p, 1);
-    if (c->lc2_nd == 3) {
-      pass(p, tl, 2);
-      LC2_CUDA(cudaMemcpyAsync(p, tl, nv * sizeof(long long), cudaMemcpyDeviceToDevice, c->stream));
-    }
+    long long* d = c->d_fd + f * nv;
+    if (box_sums(c, d, tl.p) != d)
+      LC2_CUDA(cudaMemcpyAsync(d, tl.p, nv * sizeof(long long), cudaMemcpyDeviceToDevice, c->stream));
   }
   lc2::k_fixed_centre<<<blocks, 256, 0, c->stream>>>(c->d_fs, c->d_fd, nv, (long long)c->n);
   // the solve factors, and (S_M, S_G) interleaved per voxel through the
   // 8-byte temporary into the sums' own buffer
   lc2::k_fixed_solve_static<<<blocks, 256, 0, c->stream>>>(c->d_fs, c->d_fd, nv, c->fp.thr_m,
                                                            c->fp.thr_g,
-                                                           reinterpret_cast<int2*>(tl), c->d_fsv);
-  LC2_CUDA(cudaMemcpyAsync(c->d_fs, tl, nv * sizeof(int2), cudaMemcpyDeviceToDevice, c->stream));
+                                                           reinterpret_cast<int2*>(tl.p), c->d_fsv);
+  LC2_CUDA(cudaMemcpyAsync(c->d_fs, tl.p, nv * sizeof(int2), cudaMemcpyDeviceToDevice, c->stream));
   c->launches += 3;
   LC2_CUDA(cudaGetLastError());
   LC2_CUDA(cudaStreamSynchronize(c->stream));
@@ -1668,54 +1763,38 @@ int fixed_static_sums(lc2_context* c) {
 // float operations of lc2::mi_bin, and its entropy.
 int set_static_bins(lc2_context* c) {
   const size_t nv = c->nv;
-  std::vector<float> host(nv);
   const int ustore = c->cfg.high_res_is_moving ? c->cfg.storage : LC2_STORE_F32;
-  float* tmp = c->d_scratch;  // slot 0
-  LC2_TRY(to_float(c, c->d_static, tmp, nv, ustore));
-  LC2_CUDA(cudaMemcpyAsync(host.data(), tmp, sizeof(float) * nv, cudaMemcpyDeviceToHost, c->stream));
+  float* img = c->d_scratch;  // slot 0
+  LC2_TRY(to_float(c, c->d_static, img, nv, ustore));
+  TempBuffer<unsigned long long> t;  // counts, then the range's two words
+  LC2_CUDA(t.alloc(lc2::kMiBins + 1, c->stream));
+  unsigned* range = reinterpret_cast<unsigned*>(t.p + lc2::kMiBins);
+  LC2_CUDA(cudaMemsetAsync(t.p, 0, (lc2::kMiBins + 1) * sizeof(unsigned long long), c->stream));
+  LC2_CUDA(cudaMemsetAsync(range, 0xff, sizeof(unsigned), c->stream));
+  const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 8);
+  lc2::k_mi_static_range<><<<blocks, 256, 0, c->stream>>>(img, nv, range);
+  lc2::k_mi_static_bins<><<<blocks, 256, 0, c->stream>>>(img, nv, range, c->d_sbin, t.p);
+  c->launches += 2;
+  LC2_CUDA(cudaGetLastError());
+  unsigned long long counts[lc2::kMiBins];
+  LC2_CUDA(cudaMemcpyAsync(counts, t.p, sizeof(counts), cudaMemcpyDeviceToHost, c->stream));
   LC2_CUDA(cudaStreamSynchronize(c->stream));
-  float lo = host[0], hi = host[0];
-  for (float v : host) {
-    lo = std::min(lo, v);
-    hi = std::max(hi, v);
-  }
-  const float sc = lc2::mi_scale(lo, hi);
-  std::vector<unsigned char> bins(nv);
-  std::vector<long long> counts(lc2::kMiBins, 0);
-  for (size_t i = 0; i < nv; ++i) {
-    const float t = (host[i] - lo) * sc;
-    int b = (int)std::round(t);
-    b = std::min(std::max(b, 0), lc2::kMiBins - 1);
-    bins[i] = (unsigned char)b;
-    ++counts[b];
-  }
   double s = 0.0;
-  for (long long n : counts)
+  for (unsigned long long n : counts)
     if (n) s += (double)n * std::log((double)n);
   c->h_static = std::log((double)nv) - s / (double)nv;
-  LC2_CUDA(cudaMemcpyAsync(c->d_sbin, bins.data(), nv, cudaMemcpyHostToDevice, c->stream));
-  LC2_CUDA(cudaStreamSynchronize(c->stream));
   c->ready = true;
   return LC2_OK;
 }
 
-// fmax: the fixed image's largest |value| (image_absmax).
+// Everything that depends on the fixed image (device floats), given both
+// images' largest |value|: the fixed image on the virtual grid, the fixed-point
+// parameters and the static fields.
 int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
   const int storage = c->cfg.storage;
   drop_graphs(c);  // they hold the old images' fixed-point scales
-  struct Free {
-    float* p;
-    cudaStream_t st;
-    ~Free() { dev_free(p, st); }
-  };
   // fixed volume resampled onto the virtual grid through the identity
   // (VirtualToFixed, src/Interpolator/interpolator.cu:526-528)
-  float* ffix = nullptr;
-  LC2_CUDA(dev_alloc((void**)&ffix, sizeof(float) * c->nf, c->stream));
-  Free guard2{ffix, c->stream};
-  // cudaMemcpyDefault: the fixed image is host memory (lc2_set_images) or
-  // device memory (lc2_set_images_device)
-  LC2_CUDA(cudaMemcpyAsync(ffix, fixed, sizeof(float) * c->nf, cudaMemcpyDefault, c->stream));
   lc2::Xform id{};
   {
     float ident[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
@@ -1725,7 +1804,21 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
   c->h_xf[0] = id;
   LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform), cudaMemcpyHostToDevice, c->stream));
   float* vfix = c->d_scratch;  // slot 0 as temporary
-  LC2_TRY(launch_warp(c, c->warp_nd, ffix, LC2_STORE_F32, c->cfg.fixed, c->d_xf, 0, 1, vfix, c->nv));
+  if (c->warp_nd == 3) {
+    // k_presample's samples are launch_warp's (145 us at 256^3), four times as fast
+    lc2::FusedParams S{};
+    S.mx = c->cfg.fixed.dim[0];
+    S.my = c->cfg.fixed.dim[1];
+    S.mz = c->cfg.fixed.dim[2];
+    S.vx = c->virt.dim[0];
+    S.vy = c->virt.dim[1];
+    S.vz = c->virt.dim[2];
+    LC2_CUDA(lc2::presample_launch<float>(fixed, S, c->d_xf, 0, 1, vfix, S.vx,
+                                          (size_t)S.vx * S.vy, c->nv, c->stream));
+    ++c->launches;
+  } else {
+    LC2_TRY(launch_warp(c, 2, fixed, LC2_STORE_F32, c->cfg.fixed, c->d_xf, 0, 1, vfix, c->nv));
+  }
   if (c->cfg.high_res_is_moving) {
     LC2_TRY(convert_to_storage(c, vfix, c->d_static, c->nv, storage));
   } else {
@@ -1783,23 +1876,7 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
   F.kbits = 0;
   while (((long long)(c->n + 1) << (F.kbits + 1)) <= (1LL << 30)) ++F.kbits;
   if (c->cfg.high_res_is_moving) {
-    // the ultrasound is static: its weighting factor per voxel and their sum,
-    // once, with the generic moments kernel on M = G = 0
-    float* zero = c->d_scratch;
-    LC2_CUDA(cudaMemsetAsync(zero, 0, sizeof(float) * c->nv, c->stream));
-    LC2_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long) * 2, c->stream));
-    lc2::MomentParams Q = P;
-    choose_zchunks(c, 1, Q);
-    Q.u_stride = Q.m_stride = Q.g_stride = 0;
-    if (c->lc2_nd == 3)
-      LC2_TRY(launch_moments_nd<3>(c, c->d_static, storage, zero, zero, Q, 0, 1, c->d_sigma, nullptr));
-    else
-      LC2_TRY(launch_moments_nd<2>(c, c->d_static, storage, zero, zero, Q, 0, 1, c->d_sigma, nullptr));
-    unsigned long long sums[2] = {0, 0};
-    LC2_CUDA(cudaMemcpyAsync(sums, c->d_acc, sizeof(sums), cudaMemcpyDeviceToHost, c->stream));
-    LC2_CUDA(cudaStreamSynchronize(c->stream));
-    c->sigma_sum = (long long)sums[1];
-    LC2_TRY(static_window_sum(c));
+    LC2_TRY(static_sums(c));
   } else {
     LC2_TRY(fixed_static_sums(c));
   }
@@ -1817,12 +1894,20 @@ int lc2_set_images(lc2_context* c, const float* fixed, const float* moving) {
   if (!c->owns_moving)
     return fail(LC2_ERR_INVALID_ARGUMENT, "the frames of a stack share the stack's moving volume");
   LC2_TRY(select_device(c));
-  float fmax = 0.0f, mmax = 0.0f;
-  LC2_TRY(image_absmax(fixed, c->nf, "fixed", &fmax));
-  LC2_TRY(image_absmax(moving, c->nm, "moving", &mmax));
+  // both images to the device, where they are checked
+  TempBuffer<float> f, m;
+  LC2_CUDA(f.alloc(c->nf, c->stream));
+  LC2_CUDA(m.alloc(c->nm, c->stream));
+  LC2_CUDA(cudaMemcpyAsync(f.p, fixed, sizeof(float) * c->nf, cudaMemcpyHostToDevice, c->stream));
+  LC2_CUDA(cudaMemcpyAsync(m.p, moving, sizeof(float) * c->nm, cudaMemcpyHostToDevice, c->stream));
+  float mx[2];
+  bool bad[2];
+  LC2_TRY(device_absmax(c, f.p, c->nf, m.p, c->nm, mx, bad));
+  if (bad[0]) LC2_TRY(image_absmax(fixed, c->nf, "fixed", &mx[0]));  // names the first
+  if (bad[1]) LC2_TRY(image_absmax(moving, c->nm, "moving", &mx[1]));
   c->ready = false;
-  LC2_TRY(upload_image(c, moving, c->nm, c->d_moving, c->cfg.storage));
-  return set_fixed(c, fixed, fmax, mmax);
+  LC2_TRY(convert_to_storage(c, m.p, c->d_moving, c->nm, c->cfg.storage));
+  return set_fixed(c, f.p, mx[0], mx[1]);
 }
 
 int lc2_set_images_device(lc2_context* c, const float* fixed, const float* moving) {
@@ -1841,25 +1926,14 @@ int lc2_set_images_device(lc2_context* c, const float* fixed, const float* movin
                   "lc2_set_images_device needs device memory of the context's device");
     }
   }
-  // largest |value| and NaN/Inf flag of each image, on the device
-  unsigned int* flags = reinterpret_cast<unsigned int*>(c->d_acc);  // 4 words, reset below
-  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
-  const int blocks = 152 * 4;
-  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(fixed, c->nf, flags);
-  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(moving, c->nm, flags + 2);
-  LC2_CUDA(cudaGetLastError());
-  unsigned int h[4] = {0, 0, 0, 0};
-  LC2_CUDA(cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  LC2_CUDA(cudaStreamSynchronize(c->stream));
-  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
-  if (h[1]) return fail(LC2_ERR_INVALID_ARGUMENT, "fixed image has NaN/Inf");
-  if (h[3]) return fail(LC2_ERR_INVALID_ARGUMENT, "moving image has NaN/Inf");
-  float fmax, mmax;
-  std::memcpy(&fmax, &h[0], 4);
-  std::memcpy(&mmax, &h[2], 4);
+  float mx[2];
+  bool bad[2];
+  LC2_TRY(device_absmax(c, fixed, c->nf, moving, c->nm, mx, bad));
+  if (bad[0]) return fail(LC2_ERR_INVALID_ARGUMENT, "fixed image has NaN/Inf");
+  if (bad[1]) return fail(LC2_ERR_INVALID_ARGUMENT, "moving image has NaN/Inf");
   c->ready = false;
-  LC2_TRY(upload_image(c, moving, c->nm, c->d_moving, c->cfg.storage, true));
-  return set_fixed(c, fixed, fmax, mmax);
+  LC2_TRY(convert_to_storage(c, moving, c->d_moving, c->nm, c->cfg.storage));
+  return set_fixed(c, fixed, mx[0], mx[1]);
 }
 
 }  // extern "C"
@@ -2489,7 +2563,15 @@ int lc2_stack_add_frame(lc2_stack* s, const lc2_geometry* frame, const float vir
   c->d_moving = s->d_moving;
   float fmax = 0.0f;
   int st = image_absmax(ultrasound, c->nf, "ultrasound", &fmax);
-  if (st == LC2_OK) st = set_fixed(c, ultrasound, fmax, s->mmax);
+  if (st == LC2_OK) {
+    TempBuffer<float> u;
+    cudaError_t e = u.alloc(c->nf, c->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(u.p, ultrasound, sizeof(float) * c->nf, cudaMemcpyHostToDevice, c->stream);
+    st = e == cudaSuccess ? set_fixed(c, u.p, fmax, s->mmax)
+                          : fail(e == cudaErrorMemoryAllocation ? LC2_ERR_OUT_OF_MEMORY : LC2_ERR_CUDA,
+                                 "frame upload: %s", cudaGetErrorString(e));
+  }
   if (st != LC2_OK) {
     std::string msg = g_err;
     lc2_destroy(c);

@@ -106,6 +106,44 @@ __device__ __forceinline__ float mi_sample(const TM* __restrict__ mov, const MiP
   return tile_sample<3, TM>(mov, P.mx, P.my, P.mz, T, threadIdx.x, threadIdx.y);
 }
 
+// Range of the static image: range[0] / [1] hold its ordered minimum / maximum
+// (mi_ord), 0xffffffff and 0 before.
+template <int = 0>
+__global__ void __launch_bounds__(256) k_mi_static_range(const float* __restrict__ img, size_t n,
+                                                         unsigned* __restrict__ range) {
+  unsigned lo = 0xffffffffu, hi = 0;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+    const unsigned u = mi_ord(img[i]);
+    lo = min(lo, u);
+    hi = max(hi, u);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(range, lo);
+    atomicMax(range + 1, hi);
+  }
+}
+
+// Bins of the static image in that range, and how many voxels each holds.
+template <int = 0>
+__global__ void __launch_bounds__(256) k_mi_static_bins(const float* __restrict__ img, size_t n,
+                                                        const unsigned* __restrict__ range,
+                                                        unsigned char* __restrict__ bin,
+                                                        unsigned long long* __restrict__ counts) {
+  __shared__ unsigned s_n[kMiBins];
+  s_n[threadIdx.x] = 0;  // 256 threads, 256 bins
+  __syncthreads();
+  const float lo = mi_unord(range[0]), sc = mi_scale(lo, mi_unord(range[1]));
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+    const int b = min(max(mi_bin(img[i], lo, sc), 0), kMiBins - 1);
+    bin[i] = (unsigned char)b;
+    atomicAdd(&s_n[b], 1u);
+  }
+  __syncthreads();
+  if (s_n[threadIdx.x]) atomicAdd(counts + threadIdx.x, (unsigned long long)s_n[threadIdx.x]);
+}
+
 // Range of the warped image of each transform. Grid (tiles of 32 x 8, z
 // chunks, transforms), block (32, 8).
 template <typename TM, bool BIG>
