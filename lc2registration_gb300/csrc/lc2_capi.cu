@@ -2680,7 +2680,8 @@ int lc2_stack_evaluate(lc2_stack* s, int count, const int* frame_ids, const floa
       S.P = c->fp;
       S.P.ntx = (c->virt.dim[0] + 31) / 32;
       S.P.zchunk = 1;
-      S.ntiles = S.P.ntx * ((c->virt.dim[1] + lc2::kListTY - 1) / lc2::kListTY);
+      const int trows = lc2::list_rows(c->cfg.patch_size);
+      S.ntiles = S.P.ntx * ((c->virt.dim[1] + trows - 1) / trows);
       S.count = 0;
       S.eval0 = k;
       S.pad_ = 0;
@@ -2838,7 +2839,8 @@ int lc2_merger_evaluate(lc2_merger* m, int n, lc2_context* const* ctxs, const in
     S.P = c->fp;
     S.P.ntx = (c->virt.dim[0] + 31) / 32;
     S.P.zchunk = 1;
-    S.ntiles = S.P.ntx * ((c->virt.dim[1] + lc2::kListTY - 1) / lc2::kListTY);
+    const int trows = lc2::list_rows(c->cfg.patch_size);
+    S.ntiles = S.P.ntx * ((c->virt.dim[1] + trows - 1) / trows);
     S.count = counts[i];
     S.eval0 = k;
     S.pad_ = 0;

@@ -1030,10 +1030,14 @@ cudaError_t presample_launch(const void* mov, const FusedParams& P, const Xform*
   return cudaGetLastError();
 }
 
+// The 2D window kernel in column quads (lc2_quad2d.cuh).
+template <int WND, typename T, int R, int TY>
+cudaError_t quad2d_launch_rt(const FusedLaunch& L);
+
 // Tile heights: 3D patches of radius <= 4 run 32x16 tiles (one CTA per SM),
 // 32x24 tiles (one 768-thread CTA per SM) or 32x8 tiles (two per SM); larger
-// radii only fit 32x8; 2D runs 32x32 (two 1024-thread CTAs per SM, radius
-// 4-6, launches of four CTAs per SM or more) or 32x16 tiles (four per SM).
+// radii only fit 32x8. 2D up to radius 6 runs k_quad2d on 32x32 or 32x16 tiles,
+// beyond k_fused on 32x16 tiles.
 template <int ND, int WND, typename T, int R>
 cudaError_t fused_launch_r(const FusedLaunch& L) {
   if constexpr (ND == 3 && R > 4) {
@@ -1042,14 +1046,14 @@ cudaError_t fused_launch_r(const FusedLaunch& L) {
     if (L.tile_height == 8) return fused_launch_rt<ND, WND, T, R, 8>(L);
     if (L.tile_height == 24) return fused_launch_rt<ND, WND, T, R, 24>(L);
     return fused_launch_rt<ND, WND, T, R, 16>(L);
-  } else if constexpr (R >= 4 && R <= 6) {
-    // 32-row tiles (two 1024-thread CTAs per SM, a smaller halo per pixel)
-    // where the launch has CTAs enough for the GPU: two per SM, twice over
+  } else if constexpr (R <= 6) {
+    // 32-row tiles (a smaller halo per pixel) where the launch has CTAs enough
+    // for the GPU: two per SM, twice over
     if (L.tile_height == 32 ||
         (L.tile_height != 16 && (long long)L.cnt * ((L.P.vx + 31) / 32) * ((L.P.vy + 31) / 32) >=
                                     4LL * L.sms))
-      return fused_launch_rt<ND, WND, T, R, 32>(L);
-    return fused_launch_rt<ND, WND, T, R, 16>(L);
+      return quad2d_launch_rt<WND, T, R, 32>(L);
+    return quad2d_launch_rt<WND, T, R, 16>(L);
   } else {
     return fused_launch_rt<ND, WND, T, R, 16>(L);
   }

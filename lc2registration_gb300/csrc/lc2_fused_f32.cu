@@ -2,6 +2,7 @@
 // per storage type so the instantiations compile in parallel; also the
 // self-test kernel of the warp-specialised kernel's bounded waits.
 #include "lc2_fused_ws.cuh"
+#include "lc2_quad2d.cuh"
 
 namespace lc2 {
 LC2_DEFINE_FUSED_LAUNCH(float)

@@ -3,7 +3,7 @@
 // A work list is a sequence of segments; a segment is `count` evaluations of
 // one fixed image (static ultrasound + weighting factors, its own virtual
 // grid and fixed-point scales) against one moving image. Every evaluation is
-// cut into the 32 x 16 tiles of its fixed image, and the tiles of all
+// cut into the tiles of its fixed image (list_rows), and the tiles of all
 // segments form one range of work units, so frames of uneven sizes (a
 // 2D-to-3D frame stack, src/Interpolator/interpolator.cu:1538-1775 run for
 // many frames) or 2D registrations of different sizes share one launch.
@@ -12,7 +12,7 @@
 // is found from the previous one.
 #pragma once
 
-#include "lc2_fused.cuh"
+#include "lc2_quad2d.cuh"
 
 namespace lc2 {
 
@@ -29,10 +29,24 @@ struct ListSeg {
   long long unit0;    // first work unit of the segment
 };
 
-constexpr int kListTY = 16;
+// Rows of a tile: column quads (quad_tile_2d) up to radius 6, beyond
+// fused_tile_2d's 16.
+constexpr int list_rows(int r) { return r <= 6 ? 32 : 16; }
+
+template <int R, bool QUAD = (R <= 6)>
+struct ListGeom {
+  static constexpr int TY = list_rows(R), NT = 32 * TY, CTAS = 3, ST = NT;
+  static constexpr size_t BYTES = FusedGeom<2, TY, R>::BYTES;
+};
+template <int R>
+struct ListGeom<R, true> {
+  using G = Quad2D<list_rows(R), R>;
+  static constexpr int TY = list_rows(R), NT = G::NT, CTAS = G::CTAS, ST = G::ST;
+  static constexpr size_t BYTES = G::BYTES;
+};
 
 template <int WND, typename T, int R>
-__global__ void __launch_bounds__(32 * kListTY, 3)
+__global__ void __launch_bounds__(ListGeom<R>::NT, ListGeom<R>::CTAS)
     k_fused_list(const ListSeg* __restrict__ segs, int nseg, long long units,
                  const Xform* __restrict__ xf, unsigned long long* __restrict__ acc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -59,10 +73,15 @@ __global__ void __launch_bounds__(32 * kListTY, 3)
     const int e = (int)(rel / s_seg.ntiles);
     const int tile = (int)(rel - (long long)e * s_seg.ntiles);
     const int ev = s_seg.eval0 + e;
-    long long m = fused_tile_2d<WND, T, T, kListTY, R>(
-        (const T*)s_seg.mov, (const T*)s_seg.ust, s_seg.sig, s_seg.su, s_seg.P, xf + ev, tile,
-        smem_raw, s_tile,
-        nullptr);
+    long long m;
+    if constexpr (R <= 6)
+      m = quad_tile_2d<WND, T, T, ListGeom<R>::TY, R>(
+          (const T*)s_seg.mov, (const T*)s_seg.ust, s_seg.sig, s_seg.su, s_seg.P, xf + ev, tile,
+          smem_raw, s_tile, nullptr);
+    else
+      m = fused_tile_2d<WND, T, T, ListGeom<R>::TY, R>(
+          (const T*)s_seg.mov, (const T*)s_seg.ust, s_seg.sig, s_seg.su, s_seg.P, xf + ev, tile,
+          smem_raw, s_tile, nullptr);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m += __shfl_down_sync(0xffffffffu, m, o);
     if ((tid & 31) == 0 && m != 0) atomicAdd(acc + 2 * (size_t)ev, (unsigned long long)m);
@@ -83,7 +102,7 @@ struct ListLaunch {
 
 template <int WND, typename T, int R>
 cudaError_t list_launch_r(const ListLaunch& L) {
-  using G = FusedGeom<2, kListTY, R>;
+  using G = ListGeom<R>;
   auto kern = k_fused_list<WND, T, R>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)G::BYTES);
