@@ -127,12 +127,24 @@ __device__ __forceinline__ long long quad_tile_2d(const TM* __restrict__ mov,
   }
   __syncthreads();
   if (T.inside) {
-    for (int i = tid; i < G::PW * G::PH; i += G::NT) {
+    // all of a thread's samples in flight before the first is stored (5 % of
+    // the kernel)
+    constexpr int K = (G::PW * G::PH + G::NT - 1) / G::NT;
+    float v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = min(tid + k * G::NT, G::PW * G::PH - 1);
       const int py = i / G::PW, px = i - py * G::PW;
       if constexpr (WND == 3)
-        mc[py * G::SP + px] = fused_sample_inside<TM>(mov, P, T.A, T.ib, T.fb, px, py + yb);
+        v[k] = fused_sample_inside<TM>(mov, P, T.A, T.ib, T.fb, px, py + yb);
       else
-        mc[py * G::SP + px] = fused_sample_inside2<TM>(mov, P, T.A, T.ib, T.fb, px, py + yb);
+        v[k] = fused_sample_inside2<TM>(mov, P, T.A, T.ib, T.fb, px, py + yb);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = min(tid + k * G::NT, G::PW * G::PH - 1);
+      const int py = i / G::PW, px = i - py * G::PW;
+      mc[py * G::SP + px] = v[k];
     }
   } else {
     for (int i = tid; i < G::PW * G::PH; i += G::NT) {
