@@ -1067,10 +1067,20 @@ int launch_mi(lc2_context* c, int cnt, double* out, unsigned* flag) {
   const long long work = tiles * v.dim[2] * (long long)std::min(cnt, 65535);
   P.zchunk = (int)std::max(1LL, std::min<long long>(lc2::kMiChunk, work / (8LL * c->sms)));
   const int chunks = (v.dim[2] + P.zchunk - 1) / P.zchunk;
-  // the histogram's shared table pays where a CTA's voxels are a small part
-  // of the grid (at most 0.5 %: neighbouring voxels then share few distinct
-  // bins): 256^3 2150 -> 4640 evals/s; at 96^3 (2 %) it crowded and lost
-  P.table = P.zchunk >= 16 && (long long)c->nv >= 200LL * 256 * P.zchunk;
+  // histogram CTAs per transform, one resident per SM: the fewest waves for the
+  // work of a share, plus its fixed cost (clearing and adding up 2^16 bins,
+  // about one block's worth)
+  const long long blocks = (long long)((v.dim[0] + 31) / 32) * ((v.dim[1] + 31) / 32) *
+                           ((v.dim[2] + lc2::kMiChunk - 1) / lc2::kMiChunk);
+  int shares = 1;
+  for (long long best = -1, g = 1; g <= std::min<long long>(blocks, c->sms); ++g) {
+    const long long waves = ((long long)std::min(cnt, 65535) * g + c->sms - 1) / c->sms;
+    const long long cost = waves * ((blocks + g - 1) / g + 1);
+    if (best < 0 || cost < best) {
+      best = cost;
+      shares = (int)g;
+    }
+  }
   // one launch covers at most 65535 transforms (grid z / y limit)
   for (int k0 = 0; k0 < cnt; k0 += 65535) {
     const int n = std::min(65535, cnt - k0);
@@ -1083,15 +1093,19 @@ int launch_mi(lc2_context* c, int cnt, double* out, unsigned* flag) {
       auto range = big ? lc2::k_mi_range<T, true> : lc2::k_mi_range<T, false>;
       auto hist = big ? lc2::k_mi_hist<T, true> : lc2::k_mi_hist<T, false>;
       range<<<grid, block, 0, c->stream>>>(mov, P, c->xf, k0, c->d_rmin, c->d_rmax);
-      hist<<<grid, block, 0, c->stream>>>(mov, P, c->xf, k0, c->d_sbin, c->d_rmin, c->d_rmax,
-                                          c->d_hist);
+      cudaError_t e = cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)lc2::kMiHistBytes);
+      if (e != cudaSuccess) return e;
+      hist<<<dim3(shares, n), lc2::kMiHistThreads, lc2::kMiHistBytes, c->stream>>>(
+          mov, P, c->xf, k0, c->d_sbin, c->d_rmin, c->d_rmax, c->d_hist);
+      return cudaGetLastError();
     };
     if (st == LC2_STORE_F16)
-      passes((const __half*)c->d_moving);
+      LC2_CUDA(passes((const __half*)c->d_moving));
     else if (st == LC2_STORE_BF16)
-      passes((const __nv_bfloat16*)c->d_moving);
+      LC2_CUDA(passes((const __nv_bfloat16*)c->d_moving));
     else
-      passes((const float*)c->d_moving);
+      LC2_CUDA(passes((const float*)c->d_moving));
     lc2::k_mi_part<<<dim3(lc2::kMiParts, n), 256, 0, c->stream>>>(c->d_hist, k0,
                                                                   P.warped_is_high_res, c->d_mipart);
     c->launches += 3;

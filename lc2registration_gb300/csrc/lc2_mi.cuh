@@ -32,8 +32,7 @@ struct MiParams {
   int mx, my, mz;         // warped (moving) image
   int vx, vy, vz;         // virtual grid
   int warped_is_high_res; // 1: key = static bin + 256 * warped bin; 0: the transpose
-  int zchunk;             // slices per range / histogram CTA, <= kMiChunk
-  int table;              // k_mi_hist merges counts in a shared table first
+  int zchunk;             // slices per range CTA, <= kMiChunk
 };
 
 // Order-preserving float <-> unsigned maps for atomicMin / atomicMax.
@@ -56,21 +55,19 @@ __device__ __forceinline__ int mi_bin(float v, float lo, float s) {
   return (int)roundf(__fmul_rn(__fsub_rn(v, lo), s));
 }
 
-constexpr int kMiChunk = 64;  // most slices per range / histogram CTA
+constexpr int kMiChunk = 64;  // most slices of a range CTA or histogram block
 constexpr int kMiParts = 32;  // entropy CTAs per transform (8 warped bins each)
 
-// Sampling bases of a CTA's tile for its slices [zb, ze), one per thread, in
-// shared memory, and where each slice samples (tile_where); the caller
-// synchronises.
+// Sampling base of slice zb + t (< ze) of a 32 x 8 tile, and where the slice
+// samples (tile_where), in shared memory.
 struct MiBases {
   int ib[kMiChunk][3];
   float fb[kMiChunk][3];
   float4 base[kMiChunk];
   int where[kMiChunk];
 };
-__device__ __forceinline__ void mi_bases(const Xform* X, const MiParams& P, int x0, int y0,
-                                         int zb, int ze, MiBases& B) {
-  const int t = threadIdx.y * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void mi_base(const Xform* X, const MiParams& P, int x0, int y0, int zb,
+                                        int ze, int t, MiBases& B) {
   if (zb + t < ze) {
     TileBase T;
     tile_base(X, x0, y0, zb + t, T);
@@ -86,9 +83,9 @@ __device__ __forceinline__ void mi_bases(const Xform* X, const MiParams& P, int 
 
 template <typename TM, bool BIG>
 __device__ __forceinline__ float mi_sample(const TM* __restrict__ mov, const MiParams& P,
-                                           const float* A, const MiBases& B, int t) {
+                                           const float* A, const MiBases& B, int t, float dx,
+                                           float dy) {
   const int where = B.where[t];
-  const float dx = (float)threadIdx.x, dy = (float)threadIdx.y;
   if (where == kTileInside)
     return tile_sample_inside<TM, BIG>(mov, (unsigned)P.mx, (unsigned)P.mx * (unsigned)P.my, A,
                                        B.base[t], dx, dy);
@@ -103,7 +100,7 @@ __device__ __forceinline__ float mi_sample(const TM* __restrict__ mov, const MiP
   }
 #pragma unroll
   for (int i = 0; i < 9; ++i) T.A[i] = A[i];
-  return tile_sample<3, TM>(mov, P.mx, P.my, P.mz, T, threadIdx.x, threadIdx.y);
+  return tile_sample<3, TM>(mov, P.mx, P.my, P.mz, T, (int)dx, (int)dy);
 }
 
 // Range of the static image: range[0] / [1] hold its ordered minimum / maximum
@@ -157,7 +154,7 @@ __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, Mi
   const int x0 = (blockIdx.x % ntx) * 32, y0 = (blockIdx.x / ntx) * 8;
   const int zb = blockIdx.y * P.zchunk, ze = min(zb + P.zchunk, P.vz);
   const int slot = blockIdx.z;
-  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, B);
+  mi_base(xf + k0 + slot, P, x0, y0, zb, ze, threadIdx.y * 32 + threadIdx.x, B);
   float A[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) A[i] = __ldg(&xf[k0 + slot].ah[i]);
@@ -166,7 +163,7 @@ __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, Mi
   float lo = INFINITY, hi = -INFINITY;
   if (x < P.vx && y < P.vy) {
     for (int z = zb; z < ze; ++z) {
-      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb);
+      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb, (float)threadIdx.x, (float)threadIdx.y);
       lo = fminf(lo, v);
       hi = fmaxf(hi, v);
     }
@@ -193,89 +190,81 @@ __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, Mi
   }
 }
 
-// Shared aggregation table of k_mi_hist: (key, count) slots filled by
-// open addressing; a key that finds no slot within kMiProbes probes goes
-// straight to the global histogram, so every count lands exactly once.
-constexpr int kMiTable = 2048;
-constexpr int kMiProbes = 32;
-
-__device__ __forceinline__ void mi_table_add(int* tkey, unsigned* tcnt, unsigned* h, int key,
-                                             unsigned n) {
-  int slot = (int)(((unsigned)key * 2654435761u) >> 21);  // 11-bit Fibonacci hash
-  for (int i = 0; i < kMiProbes; ++i) {
-    int k = *(volatile int*)&tkey[slot];
-    if (k == -1) {
-      k = atomicCAS(&tkey[slot], -1, key);
-      if (k == -1) k = key;  // this thread claimed the slot
-    }
-    if (k == key) {
-      atomicAdd(&tcnt[slot], n);
-      return;
-    }
-    slot = (slot + 1) & (kMiTable - 1);
-  }
-  atomicAdd(h + key, n);
-}
-
 // Joint histogram of each transform: static bins sbin (uint8 per voxel) and
-// the warped image's bins in its range. Grid and block as k_mi_range. With
-// P.table a CTA first merges its counts in a shared table (neighbouring
-// voxels share bins), then adds each key once.
+// the warped image's bins in its range. A CTA counts its share of a transform's
+// 32 x 32 x kMiChunk blocks in shared memory, all 2^16 bins as 16-bit halves of
+// 32-bit words (128 KB), and adds the non-zero ones to the global histogram at
+// the end: with global atomics per voxel (merged per warp and, on large grids, in
+// a shared table of 2048 keys) the histogram took twice the time of the same
+// sampling without it. A half that reaches 2^15 is emptied into the global bin
+// by the thread whose count crossed the mark; the CTA's other 1023 threads add
+// less than 2^15 meanwhile, so a half never overflows. Grid (shares,
+// transforms), 1024 threads.
+constexpr int kMiHistThreads = 1024;
+constexpr size_t kMiHistBytes = sizeof(unsigned) * (kMiHist / 2);
+
 template <typename TM, bool BIG>
-__global__ void __launch_bounds__(256) k_mi_hist(const TM* __restrict__ mov, MiParams P,
-                                                 const Xform* __restrict__ xf, int k0,
-                                                 const unsigned char* __restrict__ sbin,
-                                                 const unsigned* __restrict__ rmin,
-                                                 const unsigned* __restrict__ rmax,
-                                                 unsigned* __restrict__ hist) {
-  __shared__ MiBases B;
-  __shared__ int tkey[kMiTable];
-  __shared__ unsigned tcnt[kMiTable];
-  const int ntx = (P.vx + 31) / 32;
-  const int x0 = (blockIdx.x % ntx) * 32, y0 = (blockIdx.x / ntx) * 8;
-  const int zb = blockIdx.y * P.zchunk, ze = min(zb + P.zchunk, P.vz);
-  const int slot = blockIdx.z;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  const bool table = P.table != 0;
-  if (table) {
-    for (int i = tid; i < kMiTable; i += 256) {
-      tkey[i] = -1;
-      tcnt[i] = 0;
-    }
-  }
-  mi_bases(xf + k0 + slot, P, x0, y0, zb, ze, B);
+__global__ void __launch_bounds__(kMiHistThreads, 1)
+    k_mi_hist(const TM* __restrict__ mov, MiParams P, const Xform* __restrict__ xf, int k0,
+              const unsigned char* __restrict__ sbin, const unsigned* __restrict__ rmin,
+              const unsigned* __restrict__ rmax, unsigned* __restrict__ hist) {
+  extern __shared__ unsigned s_hist[];
+  __shared__ MiBases B[4];  // the block's four 32 x 8 tiles
+  const int ntx = (P.vx + 31) / 32, nty = (P.vy + 31) / 32, nzc = (P.vz + kMiChunk - 1) / kMiChunk;
+  const int slot = blockIdx.y, tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
+  const Xform* X = xf + k0 + slot;
+  for (int i = tid; i < kMiHist / 2; i += kMiHistThreads) s_hist[i] = 0;
   float A[9];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) A[i] = __ldg(&xf[k0 + slot].ah[i]);
-  __syncthreads();
-  const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-  const bool in = x < P.vx && y < P.vy;
+  for (int i = 0; i < 9; ++i) A[i] = __ldg(&X->ah[i]);
   const float lo = mi_unord(rmin[k0 + slot]), hi = mi_unord(rmax[k0 + slot]);
   const float sc = mi_scale(lo, hi);
   unsigned* h = hist + (size_t)(k0 + slot) * kMiHist;
-  const int lane = threadIdx.x;  // blockDim.x == 32: one warp per row
-  for (int z = zb; z < ze; ++z) {
-    int key = -1;
-    if (in) {
-      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb);
-      const int wb = mi_bin(v, lo, sc);
-      const int sb = sbin[((size_t)z * P.vy + y) * P.vx + x];
-      if (wb >= 0 && wb < kMiBins)
-        key = P.warped_is_high_res ? sb + kMiBins * wb : wb + kMiBins * sb;
+  const MiBases& T = B[row >> 3];
+  const float dx = (float)lane, dy = (float)(row & 7);
+  auto count = [&](int wb, int sb) {
+    if (wb < 0 || wb >= kMiBins) return;
+    const int key = P.warped_is_high_res ? sb + kMiBins * wb : wb + kMiBins * sb;
+    const int shift = 16 * (key & 1);
+    const unsigned before = atomicAdd(&s_hist[key >> 1], 1u << shift) >> shift & 0xffffu;
+    if (before == 0x7fffu) {
+      atomicSub(&s_hist[key >> 1], 0x8000u << shift);
+      atomicAdd(h + key, 0x8000u);
     }
-    // voxels of a warp that share a bin add once
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    if (key >= 0 && lane == __ffs(peers) - 1) {
-      if (table)
-        mi_table_add(tkey, tcnt, h, key, (unsigned)__popc(peers));
-      else
-        atomicAdd(h + key, (unsigned)__popc(peers));
+  };
+  for (long long blk = blockIdx.x; blk < (long long)ntx * nty * nzc; blk += gridDim.x) {
+    const int zc = (int)(blk % nzc), t = (int)(blk / nzc);
+    const int x0 = (t % ntx) * 32, y0 = (t / ntx) * 32, zb = zc * kMiChunk;
+    const int ze = min(zb + kMiChunk, P.vz);
+    __syncthreads();  // the previous block's bases are read
+    if (tid < 4 * kMiChunk) mi_base(X, P, x0, y0 + 8 * (tid / kMiChunk), zb, ze, tid % kMiChunk, B[tid / kMiChunk]);
+    __syncthreads();
+    const int x = x0 + lane, y = y0 + row;
+    if (x < P.vx && y < P.vy) {
+      const unsigned char* sb = sbin + ((size_t)zb * P.vy + y) * P.vx + x;
+      const size_t plane = (size_t)P.vx * P.vy;
+      int z = zb;
+      for (; z + 4 <= ze; z += 4) {
+        float v[4];
+        int b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          v[k] = mi_sample<TM, BIG>(mov, P, A, T, z + k - zb, dx, dy);
+          b[k] = sb[(size_t)(z + k - zb) * plane];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) count(mi_bin(v[k], lo, sc), b[k]);
+      }
+      for (; z < ze; ++z)
+        count(mi_bin(mi_sample<TM, BIG>(mov, P, A, T, z - zb, dx, dy), lo, sc),
+              sb[(size_t)(z - zb) * plane]);
     }
   }
-  if (table) {
-    __syncthreads();
-    for (int i = tid; i < kMiTable; i += 256)
-      if (tkey[i] >= 0) atomicAdd(h + tkey[i], tcnt[i]);
+  __syncthreads();
+  for (int i = tid; i < kMiHist / 2; i += kMiHistThreads) {
+    const unsigned w = s_hist[i];
+    if (w & 0xffffu) atomicAdd(h + 2 * i, w & 0xffffu);
+    if (w >> 16) atomicAdd(h + 2 * i + 1, w >> 16);
   }
 }
 
