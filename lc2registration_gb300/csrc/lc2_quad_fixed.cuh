@@ -19,7 +19,17 @@ namespace lc2 {
 //
 // Bound by the solve warps' serial chain (the moments and x pass alone take
 // 2.0 ms). 160^3, radius 3, 50 transforms: moments 3.73 ms on 16-row tiles of
-// one point per thread -> 2.98, with the resampling 4.44 -> 3.72 ms.
+// one point per thread -> 2.83 (sqrtf instead of sqrt_from: 2.99), with the
+// resampling 4.44 -> 3.35 ms. Two solving groups on alternate slices would need
+// 24 warps at 80 registers, where the moments warps spill (3.93).
+// Square root of x in [1, 2^64) from y = rsqrt.approx(x): one Newton step on
+// the exact residual x - (x y)^2 (Markstein 1990), which rounds as sqrtf does
+// (compared on every float of that range).
+__device__ __forceinline__ float sqrt_from(float x, float y) {
+  const float g = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-g, g, x), 0.5f * y, g);
+}
+
 template <int TY, int R>
 __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
     k_fixed_quad(const float* __restrict__ Ub, const int* __restrict__ Mq,
@@ -199,7 +209,7 @@ __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
   auto finish = [&]() {
 #pragma unroll
     for (int j = 0; j < kQuadOut; ++j) {
-      const float sigma = sqrtf(fuu[j]) * P.sig_scale, iu = rsqrt_ftz(fuu[j]);
+      const float iu = rsqrt_ftz(fuu[j]), sigma = sqrt_from(fuu[j], iu) * P.sig_scale;
       const float im = psv[j][0], ig = psv[j][1], rmg = psv[j][2];
       const float um = rum[j] * iu * im, ug = rug[j] * iu * ig;
       const float den = 1.0f - rmg * rmg;
