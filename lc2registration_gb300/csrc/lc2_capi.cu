@@ -1071,7 +1071,7 @@ int launch_mi(lc2_context* c, int cnt, double* out, unsigned* flag) {
   // work of a share, plus its fixed cost (clearing and adding up 2^16 bins,
   // about one block's worth)
   const long long blocks = (long long)((v.dim[0] + 31) / 32) * ((v.dim[1] + 31) / 32) *
-                           ((v.dim[2] + lc2::kMiChunk - 1) / lc2::kMiChunk);
+                           ((v.dim[2] + lc2::kMiHistChunk - 1) / lc2::kMiHistChunk);
   int shares = 1;
   for (long long best = -1, g = 1; g <= std::min<long long>(blocks, c->sms); ++g) {
     const long long waves = ((long long)std::min(cnt, 65535) * g + c->sms - 1) / c->sms;

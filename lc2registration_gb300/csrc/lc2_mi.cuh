@@ -192,15 +192,17 @@ __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, Mi
 
 // Joint histogram of each transform: static bins sbin (uint8 per voxel) and
 // the warped image's bins in its range. A CTA counts its share of a transform's
-// 32 x 32 x kMiChunk blocks in shared memory, all 2^16 bins as 16-bit halves of
+// 32 x 32 x kMiHistChunk blocks in shared memory, all 2^16 bins as 16-bit halves of
 // 32-bit words (128 KB), and adds the non-zero ones to the global histogram at
 // the end: with global atomics per voxel (merged per warp and, on large grids, in
 // a shared table of 2048 keys) the histogram took twice the time of the same
 // sampling without it. A half that reaches 2^15 is emptied into the global bin
-// by the thread whose count crossed the mark; the CTA's other 1023 threads add
-// less than 2^15 meanwhile, so a half never overflows. Grid (shares,
-// transforms), 1024 threads.
+// by the thread whose count crossed the mark; until it has, the CTA's other
+// 1023 threads add at most what is left of the block, kMiHistChunk each, so a
+// half never overflows. Grid (shares, transforms), 1024 threads.
 constexpr int kMiHistThreads = 1024;
+constexpr int kMiHistChunk = 32;
+static_assert((kMiHistThreads - 1) * kMiHistChunk < (1 << 15) && kMiHistChunk <= kMiChunk, "");
 constexpr size_t kMiHistBytes = sizeof(unsigned) * (kMiHist / 2);
 
 template <typename TM, bool BIG>
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(kMiHistThreads, 1)
               const unsigned* __restrict__ rmax, unsigned* __restrict__ hist) {
   extern __shared__ unsigned s_hist[];
   __shared__ MiBases B[4];  // the block's four 32 x 8 tiles
-  const int ntx = (P.vx + 31) / 32, nty = (P.vy + 31) / 32, nzc = (P.vz + kMiChunk - 1) / kMiChunk;
+  const int ntx = (P.vx + 31) / 32, nty = (P.vy + 31) / 32, nzc = (P.vz + kMiHistChunk - 1) / kMiHistChunk;
   const int slot = blockIdx.y, tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
   const Xform* X = xf + k0 + slot;
   for (int i = tid; i < kMiHist / 2; i += kMiHistThreads) s_hist[i] = 0;
@@ -234,10 +236,12 @@ __global__ void __launch_bounds__(kMiHistThreads, 1)
   };
   for (long long blk = blockIdx.x; blk < (long long)ntx * nty * nzc; blk += gridDim.x) {
     const int zc = (int)(blk % nzc), t = (int)(blk / nzc);
-    const int x0 = (t % ntx) * 32, y0 = (t / ntx) * 32, zb = zc * kMiChunk;
-    const int ze = min(zb + kMiChunk, P.vz);
+    const int x0 = (t % ntx) * 32, y0 = (t / ntx) * 32, zb = zc * kMiHistChunk;
+    const int ze = min(zb + kMiHistChunk, P.vz);
     __syncthreads();  // the previous block's bases are read
-    if (tid < 4 * kMiChunk) mi_base(X, P, x0, y0 + 8 * (tid / kMiChunk), zb, ze, tid % kMiChunk, B[tid / kMiChunk]);
+    if (tid < 4 * kMiHistChunk)
+      mi_base(X, P, x0, y0 + 8 * (tid / kMiHistChunk), zb, ze, tid % kMiHistChunk,
+              B[tid / kMiHistChunk]);
     __syncthreads();
     const int x = x0 + lane, y = y0 + row;
     if (x < P.vx && y < P.vy) {
