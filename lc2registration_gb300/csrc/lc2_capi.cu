@@ -310,14 +310,16 @@ __global__ void __launch_bounds__(256) k_box_line(const T* __restrict__ in, T* _
   if (line >= inner * outer) return;
   const long long g = line / inner;
   const size_t base = (size_t)g * group + (size_t)(line - g * inner);
-  const int j0 = blockIdx.y * kBoxSeg, j1 = min(j0 + kBoxSeg, len);
-  T a = 0;
-  for (int j = max(j0 - r, 0); j < min(j0 + r, len); ++j) a += in[base + (size_t)j * stride];
+  for (int j0 = blockIdx.y * kBoxSeg; j0 < len; j0 += gridDim.y * kBoxSeg) {
+    const int j1 = min(j0 + kBoxSeg, len);
+    T a = 0;
+    for (int j = max(j0 - r, 0); j < min(j0 + r, len); ++j) a += in[base + (size_t)j * stride];
 #pragma unroll 4
-  for (int j = j0; j < j1; ++j) {
-    if (j + r < len) a += in[base + (size_t)(j + r) * stride];
-    out[base + (size_t)j * stride] = a;
-    if (j - r >= 0) a -= in[base + (size_t)(j - r) * stride];
+    for (int j = j0; j < j1; ++j) {
+      if (j + r < len) a += in[base + (size_t)(j + r) * stride];
+      out[base + (size_t)j * stride] = a;
+      if (j - r >= 0) a -= in[base + (size_t)(j - r) * stride];
+    }
   }
 }
 
@@ -1263,7 +1265,7 @@ int plan_context(const lc2_config* cfg, lc2_context* c) {
   // the padded images of k_fused_quad index a slice with 32-bit byte offsets
   if (c->presample && r <= 4) {
     c->lay = lc2::pad_layout(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], r);
-    c->quad = c->lay.slice() < (size_t)1 << 29;
+    c->quad = c->lay.slice() < (size_t)1 << 28;  // 16-byte fields at 32-bit offsets
   }
   return LC2_OK;
 }
@@ -1651,7 +1653,7 @@ T* box_sums(lc2_context* c, T* a, T* b, T* out = nullptr) {
   auto line = [&](const T* src, T* dst, long long inner, long long outer, size_t stride, size_t group,
                   long long len) {
     dim3 grid((unsigned)((inner * outer + 255) / 256),
-              (unsigned)((len + lc2::kBoxSeg - 1) / lc2::kBoxSeg));
+              (unsigned)std::min<long long>((len + lc2::kBoxSeg - 1) / lc2::kBoxSeg, 65535));
     lc2::k_box_line<T><<<grid, 256, 0, c->stream>>>(src, dst, inner, outer, stride, group, (int)len, r);
     ++c->launches;
   };
