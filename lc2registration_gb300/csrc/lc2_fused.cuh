@@ -548,11 +548,10 @@ __device__ __forceinline__ long long fused_tile_2d(const TM* __restrict__ mov,
   return acc_m;
 }
 
-// CTAs per SM each variant is compiled for: 2D 16-row tiles 4, 32-row tiles
-// 2; 3D 16- and 24-row tiles 1; 3D 8-row tiles 2 up to radius 4 (beyond,
-// shared memory holds only one).
+// CTAs per SM each variant is compiled for: 2D 4; 3D 16- and 24-row tiles 1;
+// 3D 8-row tiles 2 up to radius 4 (beyond, shared memory holds only one).
 constexpr int fused_min_blocks(int nd, int ty, int r) {
-  return nd == 2 ? (ty == 32 ? 2 : 4) : (ty == 8 && r <= 4 ? 2 : 1);
+  return nd == 2 ? 4 : (ty == 8 && r <= 4 ? 2 : 1);
 }
 
 // Resample stage as a pass of its own (presampling): the moving image on the

@@ -7,6 +7,14 @@
 
 namespace lc2 {
 
+// Square root of x in [1, 2^64) from y = rsqrt.approx(x): one Newton step on
+// the exact residual x - (x y)^2 (Markstein 1990), which rounds as sqrtf does
+// (compared on every float of that range).
+__device__ __forceinline__ float sqrt_from(float x, float y) {
+  const float g = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-g, g, x), 0.5f * y, g);
+}
+
 // Per transform the ultrasound's window sums change, those of the static MR/CT
 // and its Sobel magnitude do not (FixedStatic): eight limbs per point (S_U,
 // invalid count, UU, UM, UG), no Sobel of the warped image, and the static
@@ -22,14 +30,6 @@ namespace lc2 {
 // one point per thread -> 2.83 (sqrtf instead of sqrt_from: 2.99), with the
 // resampling 4.44 -> 3.35 ms. Two solving groups on alternate slices would need
 // 24 warps at 80 registers, where the moments warps spill (3.93).
-// Square root of x in [1, 2^64) from y = rsqrt.approx(x): one Newton step on
-// the exact residual x - (x y)^2 (Markstein 1990), which rounds as sqrtf does
-// (compared on every float of that range).
-__device__ __forceinline__ float sqrt_from(float x, float y) {
-  const float g = __fmul_rn(x, y);
-  return __fmaf_rn(__fmaf_rn(-g, g, x), 0.5f * y, g);
-}
-
 template <int TY, int R>
 __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
     k_fixed_quad(const float* __restrict__ Ub, const int* __restrict__ Mq,
