@@ -829,38 +829,28 @@ int launch_presample(lc2_context* c, int k0, int n) {
 }
 
 // Transforms per presample group for a batch of cnt: at most the buffer's
-// slots, chosen so that the moments launches (tiles of ty rows, per_sm CTAs
-// resident per SM) fill whole waves of the device, by the launchers' z-split
-// cost model -- waves x (chunk + 2R + 3), summed over the groups; ties go to
-// larger groups. At 256^3 with 24-row tiles a transform has 88 tiles: groups
-// of 19 fill 11 waves of 152 SMs exactly, where groups of 32 leave every 19th
-// wave half empty (297 against 304 waves for 512 transforms). Values do not
-// depend on the grouping.
-// Rows of the grid that 24-row tiles leave over, run as one row of 16-row
-// tiles when they fit in it (1-16 rows): at 256 rows, 10 tiles of 24 and one
-// of 16 instead of 11 of 24 (3 % of the rows computed outside the grid).
-int pt_rest_rows(const lc2_context* c) {
-  const int vy = c->virt.dim[1], rest = vy % 24;
-  return (vy > 24 && rest > 0 && rest <= 16) ? rest : 0;
+// slots, chosen so that the moments launches (quad: quad_plan's; else tiles of
+// ty rows, per_sm CTAs resident per SM) fill the device, by the launchers'
+// cost models summed over the groups; ties go to larger groups. At 256^3 a
+// transform has 80 tiles of 24 rows and 8 of 16: groups of 19 fill 11 waves of
+// 152 SMs exactly. Values do not depend on the grouping.
+lc2::QuadPlan plan_quad(const lc2_context* c, int cnt) {
+  return lc2::quad_plan(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], c->cfg.patch_size, cnt, c->sms,
+                        c->zchunk);
 }
 
-int presample_group(const lc2_context* c, int cnt, int ty, int per_sm) {
+int presample_group(const lc2_context* c, int cnt, bool quad, int ty, int per_sm) {
   const int cap = c->pre_slots;
   if (cnt <= cap) return cnt;
-  const int vz = c->virt.dim[2], r = c->cfg.patch_size;
+  const int vx = c->virt.dim[0], vy = c->virt.dim[1], vz = c->virt.dim[2], r = c->cfg.patch_size;
   const long long sms = (long long)std::max(1, c->sms) * std::max(1, per_sm);
-  const long long ntx = (c->virt.dim[0] + 31) / 32;
-  // launches per group: (tiles per transform, weight = tile rows)
-  const int rest = ty == 24 ? pt_rest_rows(c) : 0;
-  const long long tiles = ntx * ((c->virt.dim[1] - rest + ty - 1) / ty);
-  auto launch_cost = [&](long long t, int n) -> long long {
-    const int zc = c->zchunk > 0 ? std::min(c->zchunk, vz) : lc2::auto_zchunk(vz, r, t * n, sms);
-    const long long chunks = (vz + zc - 1) / zc;
-    return (t * n * chunks + sms - 1) / sms * (zc + 2 * r + 3);
-  };
+  const long long tiles = (long long)((vx + 31) / 32) * ((vy + ty - 1) / ty);
   auto cost = [&](int n) -> long long {
     if (n <= 0) return 0;
-    return launch_cost(tiles, n) * ty + (rest ? launch_cost(ntx, n) * 16 : 0);
+    if (quad) return plan_quad(c, n).cost;
+    const int zc = c->zchunk > 0 ? std::min(c->zchunk, vz) : lc2::auto_zchunk(vz, r, tiles * n, sms);
+    const long long chunks = (vz + zc - 1) / zc;
+    return (tiles * n * chunks + sms - 1) / sms * (zc + 2 * r + 3);
   };
   int best_g = cap;
   long long best = -1;
@@ -915,43 +905,26 @@ int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
     LC2_TRY(ensure_presample(c, cnt));
     const bool quad = use_quad(c);
     auto moments_one = [&](const float* buf) {
-      if (quad) return lc2::quad_launch(L, buf, c->d_uq, c->d_ss, c->lay);
+      if (quad) {
+        const lc2::QuadPlan plan = plan_quad(c, L.cnt);
+        c->launches += plan.rows16;
+        return lc2::quad_launch(L, buf, c->d_uq, c->d_ss, c->lay, plan);
+      }
       if (c->cfg.storage == LC2_STORE_F16) return lc2::fused_ps_entry<__half>(L, buf);
       if (c->cfg.storage == LC2_STORE_BF16) return lc2::fused_ps_entry<__nv_bfloat16>(L, buf);
       return lc2::fused_ps_entry<float>(L, buf);
     };
     // the moments pass of a group: radius <= 4 with the in-kernel Sobel
-    // (k_fused_quad on 24-row tiles, the rows left over by them as one row of
-    // its 16-row tiles; k_fused_ps where 8/16-row tiles are asked for), else
-    // k_fused
+    // (k_fused_quad; k_fused_ps where 8/16-row tiles are asked for), else
+    // k_fused on 8-row tiles
     auto moments = [&](int j, int n, const float* buf) {
       L.k0 = k0 + j;
       L.cnt = n;
       L.pre = buf;
-      if (c->cfg.patch_size > 4) {
-        ++c->launches;
-        return fused();
-      }
-      const int rest = L.tile_height == 24 ? pt_rest_rows(c) : 0;
-      L.y_off = 0;
-      L.y_rows = c->virt.dim[1] - rest;
-      cudaError_t err = moments_one(buf);
       ++c->launches;
-      if (err == cudaSuccess && rest) {
-        L.tile_height = 16;
-        L.y_off = c->virt.dim[1] - rest;
-        L.y_rows = rest;
-        err = moments_one(buf);
-        ++c->launches;
-        L.tile_height = 24;
-      }
-      L.y_off = L.y_rows = 0;
-      return err;
+      return c->cfg.patch_size > 4 ? fused() : moments_one(buf);
     };
-    // the moments kernel's tile height: 24 (k_fused_quad), 16 (k_fused_ps) or,
-    // beyond radius 4, 8 (k_fused on presampled images)
-    const int ty = c->cfg.patch_size > 4 ? 8 : (L.tile_height == 24 ? 24 : 16);
-    const int group = presample_group(c, cnt, ty, 1);
+    const int group = presample_group(c, cnt, quad, c->cfg.patch_size > 4 ? 8 : 16, 1);
     for (int j = 0; j < cnt; j += group) {
       const int n = std::min(group, cnt - j);
       LC2_TRY(launch_presample(c, k0 + j, n));
@@ -1000,7 +973,11 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
   L.stream = c->stream;
   auto fixed = [&]() {
     TimerScope ts(c, K_MOMENTS);
-    if (use_quad(c)) return lc2::fixed_quad_launch(L, c->d_uq, c->lay);
+    if (use_quad(c)) {
+      const lc2::QuadPlan plan = plan_quad(c, L.cnt);
+      c->launches += plan.rows16;
+      return lc2::fixed_quad_launch(L, c->d_uq, c->lay, plan);
+    }
     switch (c->cfg.storage) {
       case LC2_STORE_F16: return lc2::fixed_launch<__half>(L);
       case LC2_STORE_BF16: return lc2::fixed_launch<__nv_bfloat16>(L);
@@ -1012,34 +989,17 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
     // the ultrasound resampled in a pass of its own, then the moments, in
     // groups of the presample buffer's capacity
     LC2_TRY(ensure_presample(c, cnt));
-    // the moments kernel's tile height and CTAs per SM: 24 rows
-    // (k_fixed_quad, the rows it leaves over on its 16-row tiles), else
-    // k_fused_fixed3's 16 or 8
-    const int ty = c->cfg.patch_size > 4 || L.tile_height == 8 ? 8
-                   : L.tile_height == 24                       ? 24
-                                                               : 16;
-    const int group =
-        presample_group(c, cnt, ty, ty == 24 ? 1 : lc2::fused_min_blocks(3, ty, c->cfg.patch_size));
-    const int rest = ty == 24 ? pt_rest_rows(c) : 0;
+    const int ty = c->cfg.patch_size > 4 || L.tile_height == 8 ? 8 : 16;  // k_fused_fixed3's
+    const int group = presample_group(c, cnt, use_quad(c), ty,
+                                      lc2::fused_min_blocks(3, ty, c->cfg.patch_size));
     for (int j = 0; j < cnt; j += group) {
       const int n = std::min(group, cnt - j);
       LC2_TRY(launch_presample(c, k0 + j, n));
       L.k0 = k0 + j;
       L.cnt = n;
       L.pre = c->d_pre;
-      L.y_off = 0;
-      L.y_rows = c->virt.dim[1] - rest;
       e = fixed();
       ++c->launches;
-      if (e == cudaSuccess && rest) {
-        L.tile_height = 16;
-        L.y_off = c->virt.dim[1] - rest;
-        L.y_rows = rest;
-        e = fixed();
-        ++c->launches;
-        L.tile_height = 24;
-      }
-      L.y_off = L.y_rows = 0;
       if (e != cudaSuccess)
         return fail(LC2_ERR_CUDA, "fused kernel (resampled ultrasound): %s", cudaGetErrorString(e));
     }

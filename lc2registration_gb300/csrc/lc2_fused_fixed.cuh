@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(32 * TY, fused_min_blocks(3, TY, R))
   const int tid = threadIdx.x;
   const int slot = blockIdx.x;
   const int tile = blockIdx.y;
-  const int x0 = (tile % P.ntx) * 32, y0 = P.y0 + (tile / P.ntx) * TY;
+  const int x0 = (tile % P.ntx) * 32, y0 = (tile / P.ntx) * TY;
   const Xform* X = xf + k0 + slot;
   // sampling base (x0 - R - 1, 48 floor(y0 / 48) - R - 1), as in k_fused, so
   // 8- and 16-row tiles sample every voxel identically
@@ -376,9 +376,6 @@ struct FixedLaunch {
   int sms;          // multiprocessors of the device
   cudaStream_t stream;
   const float* pre = nullptr;  // 3D: presampled ultrasound of the launch (k_presample)
-  // 3D presampled: the launch's tiles cover output rows [y_off, y_off +
-  // y_rows) (y_rows 0: the whole grid)
-  int y_off = 0, y_rows = 0;
 };
 
 template <typename T, int R, int TY, typename K>
@@ -399,10 +396,8 @@ cudaError_t fixed_launch3_k(const FixedLaunch& L, K kern) {
                                        (int)F::BYTES);
   if (e != cudaSuccess) return e;
   FusedParams P = L.P;
-  const int rows = L.y_rows > 0 ? L.y_rows : P.vy;
-  const int ntx = (P.vx + 31) / 32, nty = (rows + TY - 1) / TY;
+  const int ntx = (P.vx + 31) / 32, nty = (P.vy + TY - 1) / TY;
   P.ntx = ntx;
-  P.y0 = L.y_off;
   if (L.zchunk > 0)
     P.zchunk = L.zchunk < P.vz ? L.zchunk : P.vz;
   else

@@ -4,13 +4,12 @@
 namespace lc2 {
 
 cudaError_t quad_launch(const FusedLaunch& L, const float* M, const int* uq, const int2* ss,
-                        const PadLayout& lay) {
-  const bool tall = L.tile_height == 24;
+                        const PadLayout& lay, const QuadPlan& plan) {
   switch (L.P.r) {
-    case 1: return tall ? quad_launch_r<24, 1>(L, M, uq, ss, lay) : quad_launch_r<16, 1>(L, M, uq, ss, lay);
-    case 2: return tall ? quad_launch_r<24, 2>(L, M, uq, ss, lay) : quad_launch_r<16, 2>(L, M, uq, ss, lay);
-    case 3: return tall ? quad_launch_r<24, 3>(L, M, uq, ss, lay) : quad_launch_r<16, 3>(L, M, uq, ss, lay);
-    case 4: return tall ? quad_launch_r<24, 4>(L, M, uq, ss, lay) : quad_launch_r<16, 4>(L, M, uq, ss, lay);
+    case 1: return quad_launch_r<1>(L, M, uq, ss, lay, plan);
+    case 2: return quad_launch_r<2>(L, M, uq, ss, lay, plan);
+    case 3: return quad_launch_r<3>(L, M, uq, ss, lay, plan);
+    case 4: return quad_launch_r<4>(L, M, uq, ss, lay, plan);
   }
   return cudaErrorInvalidValue;
 }

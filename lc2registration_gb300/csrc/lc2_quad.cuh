@@ -34,7 +34,131 @@ struct QuadParams {
   int px;                 // row pitch of the padded images
   int origin;             // offset of voxel (0, 0) in a padded slice
   size_t slice, volume;   // strides of the padded images
+  int y0;                 // first output row of the launch's tiles
 };
+
+// How the tiles of a group of transforms cover the grid: 24-row tiles, and one
+// row of 16-row tiles below them or none, each in its own launch and z chunks.
+struct QuadPlan {
+  int rows24 = 0, rows16 = 0;  // rows of tiles
+  int z24 = 0, z16 = 0;        // slices per CTA
+  long long cost = 0;          // estimated duration: kQuadW24 per slice of a 24-row tile
+};
+// Times of a slice of a 24- and a 16-row tile, measured as 4 : 3.
+constexpr int kQuadW24 = 4, kQuadW16 = 3;
+
+// The plan with the least estimated duration, for one CTA per SM at a time and
+// 2R + 3 slices per CTA beside its output (the windows' run-up, filling and
+// draining). The 1-16 rows that 24-row tiles leave over go to 16-row tiles,
+// which fill the gaps of the 24-row launch's last wave, or, where that gains
+// less than 2 %, to 24-row tiles that reach beyond the grid: one transform at
+// 256^3, radius 4, takes 3 waves of 63 slices either way, and the second launch
+// costs 36 us of 398. Moments against two launches one after the other, the
+// second's chunks chosen by itself: that case 402 -> 362 us, 25 transforms at
+// 135 x 109 x 122, radius 2, 1049 -> 991.
+inline QuadPlan quad_plan(int vx, int vy, int vz, int r, int cnt, int sms, int zchunk) {
+  QuadPlan best;
+  const long long ntx = (vx + 31) / 32, h = 2 * r + 3;
+  sms = sms < 1 ? 1 : sms;
+  // duration of a CTAs of length la, then b of length lb as SMs come free
+  auto duration = [&](long long a, long long la, long long b, long long lb) {
+    const long long part = a % sms, t0 = a / sms * la, t1 = t0 + la;
+    const long long late = b / sms * lb, left = b % sms;  // whole rounds: every SM later by one
+    long long end = (part ? t1 : t0) + late;
+    if (left > sms - part)
+      end = t1 + late + lb;
+    else if (left && t0 + late + lb > end)
+      end = t0 + late + lb;
+    return end;
+  };
+  auto chunks = [&](int zc) { return (vz + zc - 1) / zc; };
+  // chunk sizes to consider for n columns
+  auto try_chunks = [&](long long n, auto f) {
+    if (zchunk > 0) return f(zchunk < vz ? zchunk : vz);
+    for (int nz = 1, last = 0; nz <= vz && nz <= 64 && (nz == 1 || n * nz <= 8LL * sms); ++nz) {
+      const int zc = (vz + nz - 1) / nz;
+      if (zc != last) f(zc);
+      last = zc;
+    }
+  };
+  auto keep = [&](int rows24, int rows16, int z24, int z16, long long cost) {
+    if (!best.z24 || cost < best.cost) best = {rows24, rows16, z24, z16, cost};
+  };
+  const int all24 = (vy + 23) / 24, rest = vy % 24;
+  const long long n24 = ntx * all24 * cnt;
+  try_chunks(n24, [&](int z24) {
+    keep(all24, 0, z24, vz, duration(n24 * chunks(z24), (z24 + h) * kQuadW24, 0, 0));
+  });
+  if (vy > 24 && rest > 0 && rest <= 16) {
+    // a second launch has to save 2 %
+    const long long n = ntx * (vy / 24) * cnt, m = ntx * cnt, bar = best.cost - best.cost / 50;
+    try_chunks(n, [&](int z24) {
+      try_chunks(m, [&](int z16) {
+        const long long d = duration(n * chunks(z24), (z24 + h) * kQuadW24, m * chunks(z16),
+                                     (z16 + h) * kQuadW16);
+        if (d < bar) keep(vy / 24, 1, z24, z16, d);
+      });
+    });
+  }
+  return best;
+}
+
+// The launches of a plan: the second one starts as SMs come free from the first
+// (programmatic dependent launch; both only read what earlier launches wrote
+// and add to the same sums) and its last CTA waits for the first one's end, so
+// that the second's end is the end of both.
+template <typename L24, typename L16>
+cudaError_t quad_launches(const FusedParams& f, const PadLayout& lay, const QuadPlan& plan, int cnt,
+                          L24 l24, L16 l16) {
+  QuadParams Q;
+  Q.f = f;
+  Q.px = lay.px;
+  Q.origin = (int)lay.origin();
+  Q.slice = lay.slice();
+  Q.volume = lay.volume();
+  Q.f.ntx = (f.vx + 31) / 32;
+  Q.f.zchunk = plan.z24;
+  Q.y0 = 0;
+  auto grid = [&](int rows) {
+    return dim3(cnt, Q.f.ntx * rows, (f.vz + Q.f.zchunk - 1) / Q.f.zchunk);
+  };
+  cudaError_t e = l24(Q, grid(plan.rows24));
+  if (e != cudaSuccess || !plan.rows16) return e;
+  Q.f.zchunk = plan.z16;
+  Q.y0 = 24 * plan.rows24;
+  return l16(Q, grid(plan.rows16));
+}
+
+// One launch of kern; after: it may start before the launch before it is done.
+template <typename... KP, typename... A>
+cudaError_t quad_launch_one(void (*kern)(KP...), dim3 grid, int threads, size_t smem,
+                            cudaStream_t stream, bool after, A... args) {
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// At the start of a CTA of 24-row tiles: the next launch may fill SMs as they
+// come free. At the end of one of 16-row tiles: the launch's last CTA stays
+// until the launch before it is done.
+__device__ __forceinline__ void quad_start() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void quad_join() {
+  if (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // ---- moments ----
 // The moments pass of a resampled MR/CT on presampled images (radius 1-4, the
@@ -246,11 +370,12 @@ __global__ void __launch_bounds__(QuadGeom<TY, R>::NT, 1)
   constexpr unsigned kmask = (1u << KB) - 1u;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const FusedParams& P = Q.f;
+  if constexpr (TY == 24) quad_start();
   // the window / solve warps come first: theirs is the longer chain, and the
   // schedulers prefer lower warps (5.81 against 6.03 ms below)
   const int tid = (int)threadIdx.x < G::CT ? threadIdx.x + G::PT : threadIdx.x - G::CT;
   const int lane = tid & 31, slot = blockIdx.x, tile = blockIdx.y;
-  const int x0 = (tile % P.ntx) * 32, y0 = P.y0 + (tile / P.ntx) * TY;
+  const int x0 = (tile % P.ntx) * 32, y0 = Q.y0 + (tile / P.ntx) * TY;
   const int zb = blockIdx.z * P.zchunk;
   const int ze = min(zb + P.zchunk, P.vz);
   const int e0 = zb - R;
@@ -592,43 +717,32 @@ __global__ void __launch_bounds__(QuadGeom<TY, R>::NT, 1)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc_m += __shfl_down_sync(0xffffffffu, acc_m, o);
   if (lane == 0) atomicAdd(acc + 2 * (size_t)(k0 + slot), (unsigned long long)acc_m);
+  if constexpr (TY != 24) quad_join();
 }
 
-template <int TY, int R>
+template <int R>
 cudaError_t quad_launch_r(const FusedLaunch& L, const float* M, const int* uq, const int2* ss,
-                          const PadLayout& lay) {
-  using G = QuadGeom<TY, R>;
+                          const PadLayout& lay, const QuadPlan& plan) {
   if (L.P.kbits != PatchConst<3, R>::K || L.P.n != PatchConst<3, R>::N)
     return cudaErrorInvalidValue;
-  auto kern = k_fused_quad<TY, R>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)G::BYTES);
-  if (e != cudaSuccess) return e;
-  QuadParams Q;
-  Q.f = L.P;
-  Q.px = lay.px;
-  Q.origin = (int)lay.origin();
-  Q.slice = lay.slice();
-  Q.volume = lay.volume();
-  FusedParams& P = Q.f;
-  const int rows = L.y_rows > 0 ? L.y_rows : P.vy;
-  const int ntx = (P.vx + 31) / 32, nty = (rows + TY - 1) / TY;
-  P.ntx = ntx;
-  P.y0 = L.y_off;
-  if (L.zchunk > 0)
-    P.zchunk = L.zchunk < P.vz ? L.zchunk : P.vz;
-  else
-    P.zchunk = auto_zchunk(P.vz, R, (long long)ntx * nty * L.cnt, (long long)L.sms);
-  const int nz = (P.vz + P.zchunk - 1) / P.zchunk;
-  dim3 grid(L.cnt, ntx * nty, nz);
-  kern<<<grid, G::NT, G::BYTES, L.stream>>>(M + lay.first(), uq + lay.first(), ss + lay.first(), Q,
-                                            L.k0, L.acc, L.out_measure);
-  return cudaGetLastError();
+  M += lay.first();
+  uq += lay.first();
+  ss += lay.first();
+  return quad_launches(
+      L.P, lay, plan, L.cnt,
+      [&](const QuadParams& Q, dim3 grid) {
+        return quad_launch_one(k_fused_quad<24, R>, grid, QuadGeom<24, R>::NT, QuadGeom<24, R>::BYTES,
+                               L.stream, false, M, uq, ss, Q, L.k0, L.acc, L.out_measure);
+      },
+      [&](const QuadParams& Q, dim3 grid) {
+        return quad_launch_one(k_fused_quad<16, R>, grid, QuadGeom<16, R>::NT, QuadGeom<16, R>::BYTES,
+                               L.stream, true, M, uq, ss, Q, L.k0, L.acc, L.out_measure);
+      });
 }
 
-// The moments pass of a group of presampled images (padded layout); tile
-// rows 24 or 16 (L.tile_height). Defined in lc2_quad.cu.
+// The moments pass of a group of presampled images (padded layout). Defined in
+// lc2_quad.cu.
 cudaError_t quad_launch(const FusedLaunch& L, const float* M, const int* uq, const int2* ss,
-                        const PadLayout& lay);
+                        const PadLayout& lay, const QuadPlan& plan);
 
 }  // namespace lc2

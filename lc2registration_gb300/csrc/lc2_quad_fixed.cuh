@@ -27,8 +27,8 @@ __device__ __forceinline__ float sqrt_from(float x, float y) {
 //
 // Bound by the solve warps' serial chain (the moments and x pass alone take
 // 2.0 ms). 160^3, radius 3, 50 transforms: moments 3.73 ms on 16-row tiles of
-// one point per thread -> 2.83 (sqrtf instead of sqrt_from: 2.99), with the
-// resampling 4.44 -> 3.35 ms. Two solving groups on alternate slices would need
+// one point per thread -> 2.58 (sqrtf instead of sqrt_from: 2.73), with the
+// resampling 4.44 -> 3.11 ms. Two solving groups on alternate slices would need
 // 24 warps at 80 registers, where the moments warps spill (3.93).
 template <int TY, int R>
 __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
@@ -41,10 +41,11 @@ __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
   constexpr unsigned kmask = (1u << KB) - 1u;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const FusedParams& P = Q.f;
+  quad_start();
   // the window / solve warps first, as in k_fused_quad
   const int tid = (int)threadIdx.x < G::CT ? threadIdx.x + G::PT : threadIdx.x - G::CT;
   const int lane = tid & 31, slot = blockIdx.x, tile = blockIdx.y;
-  const int x0 = (tile % P.ntx) * 32, y0 = P.y0 + (tile / P.ntx) * TY;
+  const int x0 = (tile % P.ntx) * 32, y0 = Q.y0 + (tile / P.ntx) * TY;
   const int zb = blockIdx.z * P.zchunk;
   const int ze = min(zb + P.zchunk, P.vz);
   const int e0 = zb - R;
@@ -273,42 +274,34 @@ __global__ void __launch_bounds__(QuadGeom<TY, R, kFixedLimbs, 3, false>::NT, 1)
   }
   finish();
   fixed_flush(acc_m, acc_s, acc + 2 * (size_t)(k0 + slot));
+  quad_join();
 }
 
-template <int TY, int R>
-cudaError_t fixed_quad_launch_r(const FixedLaunch& L, const int* q, const PadLayout& lay) {
-  using G = QuadGeom<TY, R, kFixedLimbs, 3, false>;
+template <int R>
+cudaError_t fixed_quad_launch_r(const FixedLaunch& L, const int* q, const PadLayout& lay,
+                                const QuadPlan& plan) {
+  using G24 = QuadGeom<24, R, kFixedLimbs, 3, false>;
+  using G16 = QuadGeom<16, R, kFixedLimbs, 3, false>;
   if (L.P.kbits != PatchConst<3, R>::K || L.P.n != PatchConst<3, R>::N)
     return cudaErrorInvalidValue;
-  auto kern = k_fixed_quad<TY, R>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)G::BYTES);
-  if (e != cudaSuccess) return e;
-  QuadParams Q;
-  Q.f = L.P;
-  Q.px = lay.px;
-  Q.origin = (int)lay.origin();
-  Q.slice = lay.slice();
-  Q.volume = lay.volume();
-  FusedParams& P = Q.f;
-  const int rows = L.y_rows > 0 ? L.y_rows : P.vy;
-  const int ntx = (P.vx + 31) / 32, nty = (rows + TY - 1) / TY;
-  P.ntx = ntx;
-  P.y0 = L.y_off;
-  if (L.zchunk > 0)
-    P.zchunk = L.zchunk < P.vz ? L.zchunk : P.vz;
-  else
-    P.zchunk = auto_zchunk(P.vz, R, (long long)ntx * nty * L.cnt, (long long)L.sms);
-  const int nz = (P.vz + P.zchunk - 1) / P.zchunk;
-  dim3 grid(L.cnt, ntx * nty, nz);
-  kern<<<grid, G::NT, G::BYTES, L.stream>>>(L.pre + lay.first(), q + lay.first(),
-                                            q + lay.volume() + lay.first(), L.S, Q, L.k0, L.acc);
-  return cudaGetLastError();
+  const float* pre = L.pre + lay.first();
+  const int *qm = q + lay.first(), *qg = q + lay.volume() + lay.first();
+  return quad_launches(
+      L.P, lay, plan, L.cnt,
+      [&](const QuadParams& Q, dim3 grid) {
+        return quad_launch_one(k_fixed_quad<24, R>, grid, G24::NT, G24::BYTES, L.stream, false, pre, qm,
+                               qg, L.S, Q, L.k0, L.acc);
+      },
+      [&](const QuadParams& Q, dim3 grid) {
+        return quad_launch_one(k_fixed_quad<16, R>, grid, G16::NT, G16::BYTES, L.stream, true, pre, qm,
+                               qg, L.S, Q, L.k0, L.acc);
+      });
 }
 
 // The moments pass of a group of presampled ultrasounds (padded layout); q:
 // the quantised static image and its Sobel magnitude, padded, one after the
-// other; tile rows 24 or 16 (L.tile_height). Defined in lc2_quad_fixed.cu.
-cudaError_t fixed_quad_launch(const FixedLaunch& L, const int* q, const PadLayout& lay);
+// other. Defined in lc2_quad_fixed.cu.
+cudaError_t fixed_quad_launch(const FixedLaunch& L, const int* q, const PadLayout& lay,
+                              const QuadPlan& plan);
 
 }  // namespace lc2

@@ -86,3 +86,31 @@ def test_fixed_quad_kernel_equals_16_row_kernel(dim, r):
     want = oracle_eval(case, mats[0], use_boxsum=False)
     assert abs(ref[0] - want) <= 1e-5 * abs(want)
     ctx.close()
+
+
+@pytest.mark.parametrize("hr_moving", [True, False])
+@pytest.mark.parametrize("dim,r", [((64, 40, 20), 2), ((33, 27, 20), 3), ((65, 56, 12), 4)])
+def test_batches_of_two_overlapping_launches(dim, r, hr_moving):
+    """Batches that fill the device run the rows 24-row tiles leave over in a
+    launch of their own that overlaps the first: same bits as the 16-row kernel,
+    from graphs and without, in groups and after another batch's buffers."""
+    case, mats = _case(dim, r)
+    if not hr_moving:
+        fixed = np.ascontiguousarray(case.moving[3:-3, 3:-3, 3:-3])
+        case = synth.Case("3D", case.fixed_geom, fixed, case.fixed_geom, case.fixed, [1.0, 1.0, 1.0],
+                          r, False, {}, mats[0])
+    rng = np.random.default_rng(1)
+    c = case.fixed_geom.center()
+    mats = np.stack([affine3d(rng.uniform(-4, 4, 3), rng.uniform(-3, 3, 3), center=c)
+                     for _ in range(100)])
+    ctx = make_context(case, "f32")
+    ctx.set_option(capi.OPTION_TILE_ROWS, 16)
+    ref = ctx.evaluate_batch(mats)
+    ctx.set_option(capi.OPTION_TILE_ROWS, 0)
+    for graphs in (1, 0):
+        ctx.set_option(capi.OPTION_GRAPHS, graphs)
+        for zc in (0, 5):
+            ctx.set_option(capi.OPTION_ZCHUNK, zc)
+            for n in (60, 100, 60):
+                np.testing.assert_array_equal(ctx.evaluate_batch(mats[:n]), ref[:n])
+    ctx.close()
