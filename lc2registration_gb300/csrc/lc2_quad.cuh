@@ -44,8 +44,10 @@ struct QuadPlan {
   int z24 = 0, z16 = 0;        // slices per CTA
   long long cost = 0;          // estimated duration: kQuadW24 per slice of a 24-row tile
 };
-// Times of a slice of a 24- and a 16-row tile, measured as 4 : 3.
-constexpr int kQuadW24 = 4, kQuadW16 = 3;
+// Times of a slice of a 24- and a 16-row tile: 1.84 and 1.51 us at radius 2,
+// 1.91 and 1.95 at 3 and 4 (the moments threads' serial chain is the same);
+// k_fixed_quad 1.57 and 1.38, 1.41 and 1.41, 1.74 and 1.41.
+constexpr int kQuadW24 = 12, kQuadW16 = 11;
 
 // The plan with the least estimated duration, for one CTA per SM at a time and
 // 2R + 3 slices per CTA beside its output (the windows' run-up, filling and
