@@ -303,7 +303,10 @@ __global__ void __launch_bounds__(32 * TY, fused_min_blocks(3, TY, R))
 
 // ---- 2D and 2D-to-3D: one 32 x 16 tile per CTA ----
 // Three CTAs per SM (42 registers): the solve's 64-bit work spills at the
-// 32 registers of four.
+// 32 registers of four. Bound by latency and barriers (shared memory is busy
+// about half the time). 400 x 300, radius 4, 100 transforms: 269 us with one
+// point's loads at a time -> 257; the solve's static
+// fields loaded before the passes 278 (spills), 2D quads as in k_quad2d 311.
 template <int WND, typename TM, int R>
 __global__ void __launch_bounds__(512, 3)
     k_fused_fixed2(const TM* __restrict__ mov, FixedStatic S, FusedParams P,
@@ -328,29 +331,49 @@ __global__ void __launch_bounds__(512, 3)
   }
   __syncthreads();
   const bool inside = T.inside;
-  for (int p = tid; p < G::NP; p += NT) {
-    int hy, hx;
-    halo_coord<G::HX, G::HY>(p, hy, hx);
-    const int gx = x0 - R + hx, gy = y0 - R + hy;
-    const bool pin = gx >= 0 && gx < P.vx && gy >= 0 && gy < P.vy;
-    float u = 0.0f;
-    int qm = 0, qg = 0;
-    if (inside) {
-      if constexpr (WND == 3)
-        u = fused_sample_inside<TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
-      else
-        u = fused_sample_inside2<TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
-    } else if (pin) {
-      u = fused_sample<WND, TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
+  // a thread's points B at a time, their loads all in flight before the first
+  // limb is stored
+  constexpr int MP = (G::NP + NT - 1) / NT, B = MP <= 3 ? MP : 2;
+#pragma unroll 1
+  for (int p0 = tid; p0 < G::NP; p0 += B * NT) {
+    float u[B];
+    int qm[B], qg[B];
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const int p = p0 + j * NT;
+      u[j] = 0.0f;
+      qm[j] = qg[j] = 0;
+      if (p < G::NP) {
+        int hy, hx;
+        halo_coord<G::HX, G::HY>(p, hy, hx);
+        const int gx = x0 - R + hx, gy = y0 - R + hy;
+        const bool pin = gx >= 0 && gx < P.vx && gy >= 0 && gy < P.vy;
+        if (pin) {
+          const size_t gi = (size_t)gy * P.vx + gx;
+          qm[j] = __ldg(S.q + gi);
+          qg[j] = __ldg(S.q + S.nv + gi);
+        }
+        if (inside) {
+          if constexpr (WND == 3)
+            u[j] = fused_sample_inside<TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
+          else
+            u[j] = fused_sample_inside2<TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
+        } else if (pin) {
+          u[j] = fused_sample<WND, TM>(mov, P, T.A, T.ib, T.fb, hx + 1, hy + 1);
+        }
+      }
     }
-    if (pin) {
-      const size_t gi = (size_t)gy * P.vx + gx;
-      qm = __ldg(S.q + gi);
-      qg = __ldg(S.q + S.nv + gi);
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const int p = p0 + j * NT;
+      if (p < G::NP) {
+        int hy, hx;
+        halo_coord<G::HX, G::HY>(p, hy, hx);
+        const int qu = quant(u[j], P.qu);
+        fixed_limbs(A + hy * G::HXP + hx, PA, qu, (u[j] > 1e-6f) ? 0 : 1, (long long)qu * qu,
+                    (long long)qu * qm[j], (long long)qu * qg[j], PatchConst<2, R>::K);
+      }
     }
-    const int qu = quant(u, P.qu);
-    fixed_limbs(A + hy * G::HXP + hx, PA, qu, (u > 1e-6f) ? 0 : 1, (long long)qu * qu,
-                (long long)qu * qm, (long long)qu * qg, PatchConst<2, R>::K);
   }
   __syncthreads();
   fused_xy<2, TY, R, 0, NL>(A);
