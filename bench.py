@@ -792,9 +792,9 @@ def main():
     traffic = None
     ipv = None  # thread instructions per output voxel of the fused kernel (ncu)
     captured = None
-    # the moments kernel of the tuned launch: 24-row tiles run k_fused_pt,
+    # the moments kernel of the tuned launch: 24-row tiles run k_fused_quad,
     # 8- and 16-row tiles k_fused_ps (presampled 3D form, radius <= 4)
-    kname = "k_fused_pt" if tuned[0] == 24 else "k_fused_ps"
+    kname = "k_fused_quad" if tuned[0] == 24 else "k_fused_ps"
     tfile = os.path.join(ROOT, "profiles", "k_fused_traffic.json")
     if os.path.exists(tfile) and args.patch <= 4:
         try:
@@ -876,10 +876,8 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": from_profile,
-                         "kernel": f"{kname} (moments pass"
-                                   + ("; the rows 24-row tiles leave over run on k_fused_ps"
-                                      if kname == "k_fused_pt" else "")
-                                   + "; the resample pass is kernels_ms_per_step.warp)",
+                         "kernel": f"{kname} (moments pass; the resample pass is "
+                                   "kernels_ms_per_step.warp)",
                          "launches_per_step": mom_launches,
                          "kernel_ms_per_launch": mom_ms / max(1, mom_launches),
                          "scope": "achieved and traffic are totals of the step's moments launches",

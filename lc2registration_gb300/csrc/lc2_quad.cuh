@@ -187,20 +187,23 @@ __device__ __forceinline__ void quad_join() {
 // * The images have zero borders (PadLayout), so no load has a bounds test,
 //   and each moments warp prefetches its rows into L2 kQuadAhead slices ahead:
 //   a slice takes about 2 us, hardly more than a DRAM access under load
-//   (without the prefetch 6.7 ms instead of 5.8 below).
+//   (without the prefetch 6.7 ms instead of 5.85 below).
 //
-// Bound: shared-memory wavefronts (about 3000 cycles of 4200 per slice of a
-// tile at radius 4) and, in the window / solve warps, their serial chain. The
-// register file sets the shape: 16 warps at 128 registers; 20 warps would need
-// 96, and the moments warps' window sums spill there. The previous kernel (one
-// halo point per thread with its limbs as 32-bit words, y pass and solve as
-// phases of their own on 24 warps) moved 167 words of shared memory per output
-// against about 120 and executed 603 instructions against about 330.
-// 256^3, radius 4, f16, 19 transforms: 8.31 -> 5.7 ms of moments (437 -> 300 us
-// per transform); 128^3 -> 96^3 radius 3, 100 transforms: 2606 -> 1941 us with
-// the resampling. Tried and slower there: eight output rows per solving thread
-// (13.9 ms: three warps cannot hide the reads), the x pass by the moments warps
-// (8.1), the Sobel magnitudes as a pass of their own (7.5 and 0.7 for the pass).
+// Bound: the data pipe of shared memory and L1 (82 % of its peak; about 2900
+// wavefronts of 3600 cycles per slice of a tile at radius 4). The register file
+// sets the shape: 16 warps at 128 registers; 20 warps would need 96, and the
+// moments warps' window sums spill there. The previous kernel (one halo point
+// per thread with its limbs as 32-bit words, y pass and solve as phases of
+// their own on 24 warps) took 1752 M shared-memory wavefronts for 19 transforms
+// at 256^3 against 1308 M and 603 instructions per voxel against 402.
+// 256^3, radius 4, f16, 19 transforms: 8.31 -> 5.85 ms of moments (437 -> 308 us
+// per transform); 128^3 -> 96^3 radius 3, 100 transforms: 2606 -> 1890 us with
+// the resampling. Tried and slower at 256^3: eight output rows per solving
+// thread (13.9 ms: three warps cannot hide the reads), the x pass by the moments
+// warps (8.1), the Sobel magnitudes as a pass of their own (7.5 and 0.7 for the
+// pass); both tile heights in one kernel (5.99, more spills); one CTA per SM
+// with an equal share of all columns (2.7 us per slice instead of 1.9: the
+// halos of neighbouring tiles come from DRAM when they march at different z).
 constexpr int kQuadOut = 4;  // output rows per solving thread
 
 // NL limb planes; NRING 16-byte ring entries per moments thread and slice of
