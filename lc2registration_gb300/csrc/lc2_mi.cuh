@@ -141,8 +141,12 @@ __global__ void __launch_bounds__(256) k_mi_static_bins(const float* __restrict_
   if (s_n[threadIdx.x]) atomicAdd(counts + threadIdx.x, (unsigned long long)s_n[threadIdx.x]);
 }
 
-// Range of the warped image of each transform. Grid (tiles of 32 x 8, z
-// chunks, transforms), block (32, 8).
+// Range of the warped image of each transform. Bound by the L1 lookups of its
+// gathers, eight samples of a thread in flight as in k_presample (one at a time:
+// 1028 us instead of 996 for the whole of 50 transforms at 128^3; eight instead
+// of four in the histogram's loop: 14 us more). Grid (tiles of 32 x 8, z chunks,
+// transforms), block (32, 8).
+constexpr int kMiRangeAhead = 8;
 template <typename TM, bool BIG>
 __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, MiParams P,
                                                   const Xform* __restrict__ xf, int k0,
@@ -162,8 +166,20 @@ __global__ void __launch_bounds__(256) k_mi_range(const TM* __restrict__ mov, Mi
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
   float lo = INFINITY, hi = -INFINITY;
   if (x < P.vx && y < P.vy) {
-    for (int z = zb; z < ze; ++z) {
-      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb, (float)threadIdx.x, (float)threadIdx.y);
+    const float dx = (float)threadIdx.x, dy = (float)threadIdx.y;
+    int z = zb;
+    for (; z + kMiRangeAhead <= ze; z += kMiRangeAhead) {
+      float v[kMiRangeAhead];
+#pragma unroll
+      for (int k = 0; k < kMiRangeAhead; ++k) v[k] = mi_sample<TM, BIG>(mov, P, A, B, z + k - zb, dx, dy);
+#pragma unroll
+      for (int k = 0; k < kMiRangeAhead; ++k) {
+        lo = fminf(lo, v[k]);
+        hi = fmaxf(hi, v[k]);
+      }
+    }
+    for (; z < ze; ++z) {
+      const float v = mi_sample<TM, BIG>(mov, P, A, B, z - zb, dx, dy);
       lo = fminf(lo, v);
       hi = fmaxf(hi, v);
     }
