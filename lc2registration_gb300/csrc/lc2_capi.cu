@@ -184,7 +184,7 @@ struct lc2_context {
   float* d_scratch = nullptr;  // per-slot warped image (+ Sobel when hr_moving)
   int slots = 1;
   size_t per_slot = 0;  // scratch bytes per slot
-  lc2::Xform* d_xf = nullptr;
+  lc2::Xform* d_xf = nullptr;  // cap transforms, and set_fixed's identity
   const lc2::Xform* xf = nullptr;  // what the kernels read: d_xf, or h_xf (direct_call)
   unsigned long long* d_acc = nullptr;
   double* d_out = nullptr;
@@ -192,9 +192,10 @@ struct lc2_context {
   // d_acc is all zero: k_finalize resets what it read, so only a launch whose
   // sums were not finalised (another path, an error) leaves it dirty
   bool acc_clean = false;
-  lc2::Xform* h_xf = nullptr;  // pinned staging
+  lc2::Xform* h_xf = nullptr;  // pinned staging, as d_xf
   double* h_out = nullptr;     // pinned results
-  int staged = 0;
+  int staged = 0;              // transforms of the last stage or evaluation, in h_xf
+  bool xf_stale = false;       // they are not in d_xf (upload_staged)
 
   lc2::MomentParams mp{};
   lc2::FusedParams fp{};
@@ -439,11 +440,11 @@ __global__ void k_fixed_solve_static(const int* __restrict__ s, const long long*
 // sigma_sum >= 0: the weighting-factor sum is static (precomputed), else it
 // is taken from the accumulator.
 // The sums it read are reset to zero, so a replayed batch starts from zero
-// without a memset. flag (one block): host memory set to 1 when out, host
-// memory too, is complete.
+// without a memset. host_out and flag (one block), both or neither: pinned host
+// memory that takes the values too, and is set to 1 when they are complete.
 __global__ void k_finalize(unsigned long long* __restrict__ acc, int count,
                            double* __restrict__ out, long long sigma_sum,
-                           unsigned* __restrict__ flag) {
+                           double* __restrict__ host_out, unsigned* __restrict__ flag) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < count) {
     const unsigned long long a0 = acc[2 * k], a1 = acc[2 * k + 1];
@@ -454,6 +455,7 @@ __global__ void k_finalize(unsigned long long* __restrict__ acc, int count,
     double v = m / s;
     if (isnan(v) || isinf(v)) v = 0.0;
     out[k] = v;
+    if (host_out) host_out[k] = v;
   }
   if (flag) raise_flag(flag);
 }
@@ -565,12 +567,13 @@ int ensure_capacity(lc2_context* c, int count) {
   host_free(c->h_out);
   c->d_xf = nullptr; c->d_acc = nullptr; c->d_out = nullptr; c->h_xf = nullptr; c->h_out = nullptr;
   c->cap = 0;
-  LC2_CUDA(dev_alloc((void**)&c->d_xf, sizeof(lc2::Xform) * ncap, c->stream));
+  c->staged = 0;
+  LC2_CUDA(dev_alloc((void**)&c->d_xf, sizeof(lc2::Xform) * (ncap + 1), c->stream));
   c->xf = c->d_xf;
   LC2_CUDA(dev_alloc((void**)&c->d_acc, sizeof(unsigned long long) * 2 * ncap, c->stream));
   c->acc_clean = false;
   LC2_CUDA(dev_alloc((void**)&c->d_out, sizeof(double) * ncap, c->stream));
-  LC2_CUDA(host_alloc((void**)&c->h_xf, sizeof(lc2::Xform) * ncap));
+  LC2_CUDA(host_alloc((void**)&c->h_xf, sizeof(lc2::Xform) * (ncap + 1)));
   LC2_CUDA(host_alloc((void**)&c->h_out, sizeof(double) * ncap));
   if (c->mi) {
     dev_free(c->d_hist, c->stream);
@@ -1011,8 +1014,9 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
   return LC2_OK;
 }
 
-// out, flag: where the values go, and the flag raised with them (direct_call).
-int launch_mi(lc2_context* c, int cnt, double* out, unsigned* flag) {
+// host_out, flag: pinned memory that takes the values beside d_out, and the flag
+// raised with them (direct_call), or null.
+int launch_mi(lc2_context* c, int cnt, double* host_out, unsigned* flag) {
   const lc2_geometry& v = c->virt;
   lc2::MiParams P;
   P.mx = c->cfg.moving.dim[0];
@@ -1074,8 +1078,8 @@ int launch_mi(lc2_context* c, int cnt, double* out, unsigned* flag) {
     LC2_CUDA(cudaGetLastError());
   }
   lc2::k_mi_nmi<<<(cnt + 127) / 128, 128, 0, c->stream>>>(c->d_mipart, cnt, c->h_static,
-                                                          (double)c->nv, c->d_rmin, c->d_rmax, out,
-                                                          flag);
+                                                          (double)c->nv, c->d_rmin, c->d_rmax, c->d_out,
+                                                          host_out, flag);
   ++c->launches;
   LC2_CUDA(cudaGetLastError());
   return LC2_OK;
@@ -1088,9 +1092,10 @@ int launch_group(lc2_context* c, int k0, int cnt) {
   return launch_fused_fixed(c, k0, cnt);
 }
 
-int launch_finalize(lc2_context* c, int count, double* out, unsigned* flag) {
+int launch_finalize(lc2_context* c, int count, double* host_out = nullptr,
+                    unsigned* flag = nullptr) {
   lc2::k_finalize<<<(count + 127) / 128, 128, 0, c->stream>>>(
-      c->d_acc, count, out, c->cfg.high_res_is_moving ? c->sigma_sum : -1LL, flag);
+      c->d_acc, count, c->d_out, c->cfg.high_res_is_moving ? c->sigma_sum : -1LL, host_out, flag);
   ++c->launches;
   LC2_CUDA(cudaGetLastError());
   return LC2_OK;
@@ -1244,7 +1249,7 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
     h += c->nv * (4 * sizeof(int) + 3 * sizeof(long long) + sizeof(float4));
   if (c->mi)
     h += c->nv + 64 * (sizeof(unsigned) * (lc2::kMiHist + 2) + sizeof(double) * 2 * lc2::kMiParts);
-  h += 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
+  h += sizeof(lc2::Xform) + 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
   if (c->presample)  // the presample buffer at its largest
     h += sizeof(float) * std::max(presample_voxels(c, c->quad) * (size_t)presample_cap(c, c->quad),
                                   c->nv * (size_t)presample_cap(c, false));
@@ -1777,8 +1782,10 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
     float ident2[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
     build_xform(c->warp_nd, c->virt, c->cfg.fixed, c->warp_nd == 2 ? ident2 : ident, &id);
   }
-  c->h_xf[0] = id;
-  LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform), cudaMemcpyHostToDevice, c->stream));
+  c->h_xf[c->cap] = id;  // behind the staged transforms, which stay
+  const lc2::Xform* d_id = c->d_xf + c->cap;
+  LC2_CUDA(cudaMemcpyAsync(c->d_xf + c->cap, c->h_xf + c->cap, sizeof(lc2::Xform),
+                           cudaMemcpyHostToDevice, c->stream));
   float* vfix = c->d_scratch;  // slot 0 as temporary
   if (c->warp_nd == 3) {
     // k_presample's samples are launch_warp's (145 us at 256^3), four times as fast
@@ -1789,11 +1796,11 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
     S.vx = c->virt.dim[0];
     S.vy = c->virt.dim[1];
     S.vz = c->virt.dim[2];
-    LC2_CUDA(lc2::presample_launch<float>(fixed, S, c->d_xf, 0, 1, vfix, S.vx,
+    LC2_CUDA(lc2::presample_launch<float>(fixed, S, d_id, 0, 1, vfix, S.vx,
                                           (size_t)S.vx * S.vy, c->nv, c->stream));
     ++c->launches;
   } else {
-    LC2_TRY(launch_warp(c, 2, fixed, LC2_STORE_F32, c->cfg.fixed, c->d_xf, 0, 1, vfix, c->nv));
+    LC2_TRY(launch_warp(c, 2, fixed, LC2_STORE_F32, c->cfg.fixed, d_id, 0, 1, vfix, c->nv));
   }
   if (c->cfg.high_res_is_moving) {
     LC2_TRY(convert_to_storage(c, vfix, c->d_static, c->nv, storage));
@@ -1917,26 +1924,39 @@ int lc2_set_images_device(lc2_context* c, const float* fixed, const float* movin
 namespace {
 
 // Validates the matrices and writes their per-transform affines into the
-// pinned staging buffer (no device work).
+// pinned staging buffer (no device work): they are the staged transforms from
+// here on, on the host only. A refused batch leaves those staged before.
 int stage_host(lc2_context* c, const float* matrices, int count) {
   if (count < 0 || (count > 0 && !matrices)) return fail(LC2_ERR_INVALID_ARGUMENT, "bad transforms");
+  const int mf = matrix_floats(c);
+  for (int k = 0; k < count; ++k)
+    for (int i = 0; i < mf; ++i)
+      if (!std::isfinite(matrices[(size_t)k * mf + i]))
+        return fail(LC2_ERR_INVALID_ARGUMENT, "transform %d has NaN/Inf", k);
   LC2_TRY(ensure_capacity(c, count));
   if (c->presample && !c->generic && !(c->pipeline && c->cfg.high_res_is_moving))
     LC2_TRY(ensure_presample(c, count));
-  const int mf = matrix_floats(c);
-  for (int k = 0; k < count; ++k) {
-    const float* m = matrices + (size_t)k * mf;
-    for (int i = 0; i < mf; ++i)
-      if (!std::isfinite(m[i])) return fail(LC2_ERR_INVALID_ARGUMENT, "transform %d has NaN/Inf", k);
-    build_xform(c->warp_nd, c->virt, c->cfg.moving, m, &c->h_xf[k]);
-  }
+  for (int k = 0; k < count; ++k)
+    build_xform(c->warp_nd, c->virt, c->cfg.moving, matrices + (size_t)k * mf, &c->h_xf[k]);
+  c->staged = count;
+  c->xf_stale = true;
+  return LC2_OK;
+}
+
+// The staged transforms into d_xf, if they are on the host only.
+int upload_staged(lc2_context* c) {
+  if (c->staged > 0 && c->xf_stale)
+    LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform) * c->staged,
+                             cudaMemcpyHostToDevice, c->stream));
+  c->xf_stale = false;
   return LC2_OK;
 }
 
 // Small batches skip the copy nodes of the graph: the last kernel writes the
-// values to pinned host memory and raises a flag there, which the host polls
+// values to pinned host memory too and raises a flag there, which the host polls
 // (one block: at most 128 values), and a single transform is read by the
-// kernels from the pinned staging buffer. One transform per call, 2D 256^2: 29.5 -> 18.0 us;
+// kernels from the pinned staging buffer (lc2_launch_staged uploads it if it
+// is launched again, xf_stale). One transform per call, 2D 256^2: 29.5 -> 18.0 us;
 // 128^3 -> 96^3: 54 -> 48 us.
 bool direct_call(const lc2_context* c, int count) { return count <= 128 && !c->pipeline; }
 unsigned* done_flag(lc2_context* c) { return reinterpret_cast<unsigned*>(c->h_err) + 8; }
@@ -1949,7 +1969,7 @@ int enqueue_batch(lc2_context* c, int count) {
   else
     LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform) * count, cudaMemcpyHostToDevice,
                              c->stream));
-  double* out = direct ? c->h_out : c->d_out;
+  double* out = direct ? c->h_out : nullptr;
   unsigned* flag = direct ? done_flag(c) : nullptr;
   // no memset: the sums start at zero (acc_clean, checked before each replay)
   int st = c->mi ? launch_mi(c, count, out, flag) : launch_group(c, 0, count);
@@ -2023,11 +2043,7 @@ int lc2_stage_transforms(lc2_context* c, const float* matrices, int count) {
   LC2_TRY(check_ctx(c));
   LC2_TRY(select_device(c));
   LC2_TRY(stage_host(c, matrices, count));
-  if (count > 0)
-    LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform) * count, cudaMemcpyHostToDevice,
-                             c->stream));
-  c->staged = count;
-  return LC2_OK;
+  return upload_staged(c);
 }
 
 int lc2_launch_staged(lc2_context* c, int count) {
@@ -2036,9 +2052,10 @@ int lc2_launch_staged(lc2_context* c, int count) {
     return fail(LC2_ERR_INVALID_ARGUMENT, "launch of %d transforms but %d staged", count, c->staged);
   if (count == 0) return LC2_OK;
   LC2_TRY(select_device(c));
+  LC2_TRY(upload_staged(c));
   c->acc_clean = false;
   LC2_TRY(clear_sums(c));
-  if (c->mi) return launch_mi(c, count, c->d_out, nullptr);
+  if (c->mi) return launch_mi(c, count, nullptr, nullptr);
   // the fused paths keep nothing per transform on the device, so one launch
   // covers the whole batch; the generic path is bounded by its scratch slots
   const int group = c->generic ? c->slots : count;
@@ -2046,7 +2063,7 @@ int lc2_launch_staged(lc2_context* c, int count) {
     int cnt = std::min(group, count - k0);
     LC2_TRY(launch_group(c, k0, cnt));
   }
-  return launch_finalize(c, count, c->d_out, nullptr);
+  return launch_finalize(c, count);
 }
 
 int lc2_fetch_results(lc2_context* c, double* out, int count) {
@@ -2073,12 +2090,12 @@ int lc2_evaluate_batch(lc2_context* c, const float* matrices, int count, double*
   if (!c->generic && c->use_graphs && !c->timing && count > 0) {
     LC2_TRY(select_device(c));
     LC2_TRY(stage_host(c, matrices, count));
-    c->staged = count;
     if (!c->acc_clean) LC2_TRY(clear_sums(c));
     c->acc_clean = false;  // until this batch is known to have finished
     const bool direct = direct_call(c, count);
     if (direct) __atomic_store_n(done_flag(c), 0u, __ATOMIC_RELAXED);
     LC2_TRY(launch_batch_graph(c, count));
+    c->xf_stale = direct && count == 1;  // else the graph uploads them
     if (!direct || !wait_flag(done_flag(c))) LC2_CUDA(cudaStreamSynchronize(c->stream));
     c->acc_clean = true;  // the batch reset every sum it used
     LC2_TRY(check_pipeline(c));
@@ -2118,7 +2135,7 @@ int lc2_evaluate_fields(lc2_context* c, const float* matrix, double* lc2_out, fl
     // LC2 and measures from the fused kernel; M and G from the generic
     // resample/Sobel kernels; sigma is the precomputed static map
     LC2_TRY(launch_fused(c, 0, 1, omeas));
-    LC2_TRY(launch_finalize(c, 1, c->d_out, nullptr));
+    LC2_TRY(launch_finalize(c, 1));
     float* w0 = c->d_scratch;
     LC2_TRY(launch_warp(c, c->warp_nd, c->d_moving, c->cfg.storage, c->cfg.moving, c->d_xf, 0, 1,
                         w0, nv));
@@ -2127,7 +2144,7 @@ int lc2_evaluate_fields(lc2_context* c, const float* matrix, double* lc2_out, fl
                              c->stream));
   } else {
     LC2_TRY(launch_group_generic(c, 0, 1, osig, omeas));
-    LC2_TRY(launch_finalize(c, 1, c->d_out, nullptr));
+    LC2_TRY(launch_finalize(c, 1));
   }
   float* w = c->d_scratch;
   const bool hrm = c->cfg.high_res_is_moving != 0;
@@ -2188,7 +2205,7 @@ int lc2_weighting_map(lc2_context* c, const float* matrix, double* lc2_out, floa
   } else {
     LC2_TRY(launch_group_generic(c, 0, 1, osig, omeas));
   }
-  LC2_TRY(launch_finalize(c, 1, c->d_out, nullptr));
+  LC2_TRY(launch_finalize(c, 1));
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
   lc2::k_weight_map<<<blocks, 256, 0, c->stream>>>(omeas, sig, nv, dmap);
   ++c->launches;

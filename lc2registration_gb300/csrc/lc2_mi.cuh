@@ -336,10 +336,11 @@ __global__ void __launch_bounds__(256) k_mi_part(unsigned* __restrict__ hist, in
 
 // NMI of each transform from its parts, summed in part order.
 // h_static: entropy of the static image; voxels: virtual-grid size. The ranges
-// are reset for the next batch; flag as in k_finalize.
+// are reset for the next batch; host_out and flag as in k_finalize.
 __global__ void k_mi_nmi(const double* __restrict__ part, int cnt, double h_static,
                          double voxels, unsigned* __restrict__ rmin, unsigned* __restrict__ rmax,
-                         double* __restrict__ out, unsigned* __restrict__ flag) {
+                         double* __restrict__ out, double* __restrict__ host_out,
+                         unsigned* __restrict__ flag) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < cnt) {
     double a = 0.0, b = 0.0;
@@ -355,6 +356,7 @@ __global__ void k_mi_nmi(const double* __restrict__ part, int cnt, double h_stat
     rmin[k] = 0xffffffffu;
     rmax[k] = 0u;
     out[k] = v;
+    if (host_out) host_out[k] = v;
   }
   if (flag) raise_flag(flag);
 }
