@@ -873,11 +873,16 @@ __global__ void __launch_bounds__(kNT) k_moments(const TU* __restrict__ Ubase,
   flush_sums(acc_m, acc_s, acc + 2 * (size_t)(k0 + slot));
 }
 
-// Raises a flag in pinned host memory after everything the block wrote there.
+// Raises a flag in pinned host memory after everything the block wrote there: the
+// barrier orders the block's writes before the raising thread's fence, and the
+// fence, between them and that thread's store, makes the store a release to the
+// host.
 __device__ __forceinline__ void raise_flag(unsigned* flag) {
-  __threadfence_system();
   __syncthreads();
-  if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned*>(flag) = 1u;
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned*>(flag) = 1u;
+  }
 }
 
 // float -> storage type conversion of a device buffer
