@@ -261,11 +261,18 @@ __device__ __forceinline__ float trilinear(const TM* __restrict__ mov, unsigned 
   return fmaf(rx, r - l, l);
 }
 
+// Limits within which a region's corners tell where its samples lie. The corners
+// and the samples each take a few roundings of offsets from the region's base, less
+// than 0.01 voxel in all where those stay within kRegionSpan; adding the base's
+// position rounds to 2^-24 of it, so the far end's limit gives way with the axis
+// (a fixed 0.01 voxel passes samples beyond the last voxel of axes of 10^5).
+constexpr float kRegionSpan = 4096.0f;
+__device__ __forceinline__ float region_end(float end) { return fmaf(end, 0.999999f, -0.01f); }
+
 // Where the samples of a 32 x 8 tile slice from base T lie: strictly inside the
 // moving volume (0 <= floor, floor + 1 <= dim - 1 on each axis), all outside
-// along some axis, or neither; kTileAny also where a coordinate may be beyond
-// floor_split's range. The tile's corners bound the affine image, 0.01 voxel
-// covers float rounding.
+// along some axis, or neither; kTileAny where it spans more than kRegionSpan (and
+// so may leave floor_split's range). The tile's corners bound the affine image.
 enum { kTileAny = 0, kTileInside = 1, kTileOutside = 2, kTileEdge = 3 };
 __device__ __forceinline__ int tile_where(const TileBase& T, int mx, int my, int mz) {
   const int dims[3] = {mx, my, mz};
@@ -276,9 +283,9 @@ __device__ __forceinline__ int tile_where(const TileBase& T, int mx, int my, int
     const float lo = T.fb[a] + fminf(ex, 0.0f) + fminf(ey, 0.0f);
     const float hi = T.fb[a] + fmaxf(ex, 0.0f) + fmaxf(ey, 0.0f);
     const float l = (float)T.ib[a] + lo, h = (float)T.ib[a] + hi, end = (float)(dims[a] - 1);
-    in = in && (l >= 0.01f) && (h <= end - 0.01f);
+    in = in && (l >= 0.01f) && (h <= region_end(end));
     out = out || (h < -0.01f - 1e-6f * fabsf(h)) || (l > end + 0.01f + 1e-6f * end);
-    near = near && (lo > -2097152.0f) && (hi < 2097152.0f);
+    near = near && (lo > -kRegionSpan) && (hi < kRegionSpan);
   }
   return !near ? kTileAny : in ? kTileInside : out ? kTileOutside : kTileEdge;
 }
