@@ -189,9 +189,10 @@ struct lc2_context {
   unsigned long long* d_acc = nullptr;
   double* d_out = nullptr;
   int cap = 0;  // capacity of d_xf/d_acc/d_out (transforms)
-  // d_acc is all zero: k_finalize resets what it read, so only a launch whose
-  // sums were not finalised (another path, an error) leaves it dirty
-  bool acc_clean = false;
+  // transforms whose sums (d_acc; d_hist, d_rmin, d_rmax) are at their start
+  // values: the last kernels of a batch reset what they read, so only new buffers
+  // and a launch whose sums were not finalised (another path, an error) are not
+  int clean = 0;
   lc2::Xform* h_xf = nullptr;  // pinned staging, as d_xf
   double* h_out = nullptr;     // pinned results
   int staged = 0;              // transforms of the last stage or evaluation, in h_xf
@@ -571,7 +572,7 @@ int ensure_capacity(lc2_context* c, int count) {
   LC2_CUDA(dev_alloc((void**)&c->d_xf, sizeof(lc2::Xform) * (ncap + 1), c->stream));
   c->xf = c->d_xf;
   LC2_CUDA(dev_alloc((void**)&c->d_acc, sizeof(unsigned long long) * 2 * ncap, c->stream));
-  c->acc_clean = false;
+  c->clean = 0;
   LC2_CUDA(dev_alloc((void**)&c->d_out, sizeof(double) * ncap, c->stream));
   LC2_CUDA(host_alloc((void**)&c->h_xf, sizeof(lc2::Xform) * (ncap + 1)));
   LC2_CUDA(host_alloc((void**)&c->h_out, sizeof(double) * ncap));
@@ -675,7 +676,7 @@ int launch_sobel(lc2_context* c, const float* in, float* out, int cnt, size_t sl
 template <int ND, typename TU>
 int launch_moments_t(lc2_context* c, const TU* U, const float* M, const float* G,
                      const lc2::MomentParams& P, int k0, int cnt, float* osig, float* omeas) {
-  c->acc_clean = false;
+  c->clean = 0;
   const lc2_geometry& v = c->virt;
   size_t smem = lc2::mom_smem_bytes(P.r);
   LC2_CUDA(cudaFuncSetAttribute(lc2::k_moments<ND, TU>,
@@ -868,7 +869,7 @@ int presample_group(const lc2_context* c, int cnt, bool quad, int ty, int per_sm
 }
 
 int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
-  c->acc_clean = false;
+  c->clean = 0;
   if (!c->cfg.high_res_is_moving || !c->d_sigma || !c->d_su)
     return fail(LC2_ERR_INVALID_ARGUMENT, "the static-ultrasound kernel needs a context with "
                 "HighResolutionModality: Moving");
@@ -952,7 +953,7 @@ int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
 // joint histogram, entropies; results straight into d_out.
 // The fused kernel of a resampled ultrasound: one launch for `cnt` transforms.
 int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
-  c->acc_clean = false;
+  c->clean = 0;
   if (c->cfg.high_res_is_moving || !c->d_fq || !c->d_fs || !c->d_fd)
     return fail(LC2_ERR_INVALID_ARGUMENT, "the resampled-ultrasound kernel needs a context with "
                 "HighResolutionModality: Fixed");
@@ -1101,18 +1102,22 @@ int launch_finalize(lc2_context* c, int count, double* host_out = nullptr,
   return LC2_OK;
 }
 
-// The device sums a batch accumulates into, zeroed for every transform the
-// buffers hold. A batch leaves them zeroed (k_finalize, k_mi_part, k_mi_nmi), so
-// this is needed only where one did not finish (acc_clean).
-int clear_sums(lc2_context* c) {
-  const size_t n = (size_t)c->cap;
+// Before a batch of count transforms: the sums it accumulates into at their start
+// values. A batch leaves them so (k_finalize, k_mi_part, k_mi_nmi); the context
+// forgets it until the caller knows that this one does.
+int clear_sums(lc2_context* c, int count) {
+  const int k0 = c->clean;
+  c->clean = 0;
+  if (k0 >= count) return LC2_OK;
+  const size_t n = (size_t)(count - k0);
   if (!c->mi) {
-    LC2_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long) * 2 * n, c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_acc + 2 * k0, 0, sizeof(unsigned long long) * 2 * n, c->stream));
     return LC2_OK;
   }
-  LC2_CUDA(cudaMemsetAsync(c->d_rmin, 0xff, sizeof(unsigned) * n, c->stream));
-  LC2_CUDA(cudaMemsetAsync(c->d_rmax, 0x00, sizeof(unsigned) * n, c->stream));
-  LC2_CUDA(cudaMemsetAsync(c->d_hist, 0, sizeof(unsigned) * lc2::kMiHist * n, c->stream));
+  LC2_CUDA(cudaMemsetAsync(c->d_rmin + k0, 0xff, sizeof(unsigned) * n, c->stream));
+  LC2_CUDA(cudaMemsetAsync(c->d_rmax + k0, 0x00, sizeof(unsigned) * n, c->stream));
+  LC2_CUDA(cudaMemsetAsync(c->d_hist + (size_t)k0 * lc2::kMiHist, 0,
+                           sizeof(unsigned) * lc2::kMiHist * n, c->stream));
   return LC2_OK;
 }
 
@@ -1671,7 +1676,7 @@ int static_sums(lc2_context* c) {
   }
   box_sums(c, q, tq, c->d_su);
   const long long* sums = box_sums(c, w.p, tw.p);
-  c->acc_clean = false;
+  c->clean = 0;
   LC2_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long), c->stream));
   lc2::k_sigma<<<blocks, 256, 0, c->stream>>>(c->d_su, sums, nx, ny, nz, r, c->lc2_nd == 3 ? r : 0,
                                               (long long)c->n, c->mp.thr_var, c->mp.sig_scale,
@@ -1971,7 +1976,7 @@ int enqueue_batch(lc2_context* c, int count) {
                              c->stream));
   double* out = direct ? c->h_out : nullptr;
   unsigned* flag = direct ? done_flag(c) : nullptr;
-  // no memset: the sums start at zero (acc_clean, checked before each replay)
+  // no memset: the sums start at zero (clear_sums, before each replay)
   int st = c->mi ? launch_mi(c, count, out, flag) : launch_group(c, 0, count);
   if (st == LC2_OK && !c->mi) st = launch_finalize(c, count, out, flag);
   c->xf = c->d_xf;
@@ -2053,17 +2058,20 @@ int lc2_launch_staged(lc2_context* c, int count) {
   if (count == 0) return LC2_OK;
   LC2_TRY(select_device(c));
   LC2_TRY(upload_staged(c));
-  c->acc_clean = false;
-  LC2_TRY(clear_sums(c));
-  if (c->mi) return launch_mi(c, count, nullptr, nullptr);
-  // the fused paths keep nothing per transform on the device, so one launch
-  // covers the whole batch; the generic path is bounded by its scratch slots
-  const int group = c->generic ? c->slots : count;
-  for (int k0 = 0; k0 < count; k0 += group) {
-    int cnt = std::min(group, count - k0);
-    LC2_TRY(launch_group(c, k0, cnt));
+  const int clean = std::max(c->clean, count);
+  LC2_TRY(clear_sums(c, count));
+  if (c->mi) {
+    LC2_TRY(launch_mi(c, count, nullptr, nullptr));
+  } else {
+    // the fused paths keep nothing per transform on the device, so one launch
+    // covers the whole batch; the generic path is bounded by its scratch slots
+    const int group = c->generic ? c->slots : count;
+    for (int k0 = 0; k0 < count; k0 += group)
+      LC2_TRY(launch_group(c, k0, std::min(group, count - k0)));
+    LC2_TRY(launch_finalize(c, count));
   }
-  return launch_finalize(c, count);
+  c->clean = clean;  // in stream order
+  return LC2_OK;
 }
 
 int lc2_fetch_results(lc2_context* c, double* out, int count) {
@@ -2090,14 +2098,14 @@ int lc2_evaluate_batch(lc2_context* c, const float* matrices, int count, double*
   if (!c->generic && c->use_graphs && !c->timing && count > 0) {
     LC2_TRY(select_device(c));
     LC2_TRY(stage_host(c, matrices, count));
-    if (!c->acc_clean) LC2_TRY(clear_sums(c));
-    c->acc_clean = false;  // until this batch is known to have finished
+    const int clean = std::max(c->clean, count);
+    LC2_TRY(clear_sums(c, count));
     const bool direct = direct_call(c, count);
     if (direct) __atomic_store_n(done_flag(c), 0u, __ATOMIC_RELAXED);
     LC2_TRY(launch_batch_graph(c, count));
     c->xf_stale = direct && count == 1;  // else the graph uploads them
     if (!direct || !wait_flag(done_flag(c))) LC2_CUDA(cudaStreamSynchronize(c->stream));
-    c->acc_clean = true;  // the batch reset every sum it used
+    c->clean = clean;  // the batch is known to have finished
     LC2_TRY(check_pipeline(c));
     std::memcpy(out, c->h_out, sizeof(double) * count);
     return LC2_OK;

@@ -46,3 +46,53 @@ def test_fetch_and_launch_after_an_evaluation(mode, r, count):
     with pytest.raises(capi.LC2Error, match="staged"):
         ctx.launch(count + 1)
     ctx.close()
+
+
+@pytest.mark.parametrize("mode,r", [("2D", 3), ("3D", 2), ("3D", 0)])
+def test_sums_between_batches_of_any_size(mode, r):
+    """Staged launches and evaluations in any order of sizes, past the buffers'
+    first 64 transforms, with kernel timing and without graphs: the sums each
+    starts from are those the one before left."""
+    case = _case(mode, r)
+    mats = perturbed(case, np.random.default_rng(3), 150)
+    ctx = make_context(case)
+    ref = [ctx.evaluate(m) for m in mats]
+    for k, count in enumerate((3, 64, 150, 1, 149, 65, 150)):
+        ctx.stage(mats[:count])
+        for _ in range(2):
+            ctx.launch(count)
+        ctx.launch(count // 2)
+        np.testing.assert_array_equal(ctx.fetch(count), ref[:count])
+        ctx.set_option(capi.OPTION_GRAPHS, k % 2)
+        ctx.enable_kernel_timing(k % 3 == 0)
+        np.testing.assert_array_equal(ctx.evaluate_batch(mats[:count]), ref[:count])
+        if r:
+            ctx.weighting_map(mats[0])
+    ctx.close()
+
+
+def test_staged_launch_does_not_pay_for_larger_batches():
+    """One transform of mutual information after a batch of 4096 (1 GiB of
+    histograms): no slower than before it but for the noise of the host's
+    clock; clearing them all takes 150 us or more."""
+    import time
+
+    case = _case("3D", 0)
+    mats = perturbed(case, np.random.default_rng(1), 1).repeat(4096, axis=0)
+    ctx = make_context(case)
+
+    def one():
+        best = 1e9
+        for _ in range(50):
+            t0 = time.perf_counter()
+            ctx.stage(mats[:1])
+            ctx.launch(1)
+            ctx.fetch(1)
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    one()
+    before = one()
+    ctx.evaluate_batch(mats)
+    assert one() < before + 60e-6
+    ctx.close()
