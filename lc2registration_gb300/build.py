@@ -23,7 +23,7 @@ SOURCES = ["lc2_capi.cu", "lc2_fused_f32.cu", "lc2_fused_f16.cu", "lc2_fused_bf1
            "lc2_export.cu", "lc2_optim.cpp", "lc2_serve.cpp", "lc2_stack_reg.cpp"]
 DEPS = SOURCES + ["lc2_kernels.cuh", "lc2_fused.cuh", "lc2_fused_ws.cuh", "lc2_list.cuh",
                    "lc2_mi.cuh", "lc2_fused_fixed.cuh", "lc2_fused_ps.cuh",
-                   "lc2_quad.cuh", "lc2_quad_fixed.cuh", "lc2_quad2d.cuh"]
+                   "lc2_quad.cuh", "lc2_quad_fixed.cuh", "lc2_quad2d.cuh", "lc2_quad_plan.hpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

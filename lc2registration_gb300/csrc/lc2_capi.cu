@@ -832,40 +832,32 @@ int launch_presample(lc2_context* c, int k0, int n) {
   return LC2_OK;
 }
 
-// Transforms per presample group for a batch of cnt: at most the buffer's
-// slots, chosen so that the moments launches (quad: quad_plan's; else tiles of
-// ty rows, per_sm CTAs resident per SM) fill the device, by the launchers'
-// cost models summed over the groups; ties go to larger groups. At 256^3 a
-// transform has 80 tiles of 24 rows and 8 of 16: groups of 19 fill 11 waves of
-// 152 SMs exactly. Values do not depend on the grouping.
-lc2::QuadPlan plan_quad(const lc2_context* c, int cnt) {
-  return lc2::quad_plan(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], c->cfg.patch_size, cnt, c->sms,
-                        c->zchunk);
+lc2::QuadPlanner quad_planner(const lc2_context* c) {
+  return lc2::QuadPlanner(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], c->cfg.patch_size, c->sms,
+                          c->zchunk);
 }
 
+// Transforms per presample group for a batch of cnt: at most the buffer's
+// slots, chosen so that the moments launches (quad: QuadPlanner's; else tiles of
+// ty rows, per_sm CTAs resident per SM) fill the device, by the launchers'
+// cost models summed over the groups. At 256^3 a transform has 88 tiles of 24
+// rows: groups of 19 fill 11 waves of 152 SMs exactly. Values do not depend on
+// the grouping.
 int presample_group(const lc2_context* c, int cnt, bool quad, int ty, int per_sm) {
   const int cap = c->pre_slots;
   if (cnt <= cap) return cnt;
+  if (quad) {
+    const lc2::QuadPlanner planner = quad_planner(c);
+    return lc2::group_size(cnt, cap, [&](int n) { return planner.plan(n).cost; });
+  }
   const int vx = c->virt.dim[0], vy = c->virt.dim[1], vz = c->virt.dim[2], r = c->cfg.patch_size;
   const long long sms = (long long)std::max(1, c->sms) * std::max(1, per_sm);
   const long long tiles = (long long)((vx + 31) / 32) * ((vy + ty - 1) / ty);
-  auto cost = [&](int n) -> long long {
-    if (n <= 0) return 0;
-    if (quad) return plan_quad(c, n).cost;
+  return lc2::group_size(cnt, cap, [&](int n) -> long long {
     const int zc = c->zchunk > 0 ? std::min(c->zchunk, vz) : lc2::auto_zchunk(vz, r, tiles * n, sms);
     const long long chunks = (vz + zc - 1) / zc;
     return (tiles * n * chunks + sms - 1) / sms * (zc + 2 * r + 3);
-  };
-  int best_g = cap;
-  long long best = -1;
-  for (int g = cap; g >= (cap + 1) / 2; --g) {
-    const long long total = (long long)(cnt / g) * cost(g) + cost(cnt % g);
-    if (best < 0 || total < best) {
-      best = total;
-      best_g = g;
-    }
-  }
-  return best_g;
+  });
 }
 
 int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
@@ -910,7 +902,7 @@ int launch_fused(lc2_context* c, int k0, int cnt, float* omeas) {
     const bool quad = use_quad(c);
     auto moments_one = [&](const float* buf) {
       if (quad) {
-        const lc2::QuadPlan plan = plan_quad(c, L.cnt);
+        const lc2::QuadPlan plan = quad_planner(c).plan(L.cnt);
         c->launches += plan.rows16;
         return lc2::quad_launch(L, buf, c->d_uq, c->d_ss, c->lay, plan);
       }
@@ -978,7 +970,7 @@ int launch_fused_fixed(lc2_context* c, int k0, int cnt) {
   auto fixed = [&]() {
     TimerScope ts(c, K_MOMENTS);
     if (use_quad(c)) {
-      const lc2::QuadPlan plan = plan_quad(c, L.cnt);
+      const lc2::QuadPlan plan = quad_planner(c).plan(L.cnt);
       c->launches += plan.rows16;
       return lc2::fixed_quad_launch(L, c->d_uq, c->lay, plan);
     }

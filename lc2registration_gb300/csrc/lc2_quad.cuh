@@ -2,32 +2,9 @@
 #pragma once
 
 #include "lc2_fused.cuh"
+#include "lc2_quad_plan.hpp"
 
 namespace lc2 {
-
-// Presampled images and the static ultrasound's fields in the layout
-// k_fused_quad reads: every image has a border of zeros wide enough for the
-// halo and the Sobel margin of every tile, so the kernel's loads need no bounds
-// test. All have the same strides, so one offset addresses them all.
-struct PadLayout {
-  int px, py, pz;   // padded extents (px: row pitch)
-  int b;            // border voxels before x = 0, y = 0 and z = 0
-  size_t slice() const { return (size_t)px * py; }
-  size_t volume() const { return slice() * pz; }
-  size_t first() const { return slice() * b; }          // of slice 0
-  size_t origin() const { return (size_t)px * b + b; }  // of voxel (0, 0) in a slice
-};
-
-// Border r + 1 before, and after the last tile (x: whole 32-column tiles; y:
-// the last row any tile's quads touch); z: slices -r-1 .. vz+r+1.
-inline PadLayout pad_layout(int vx, int vy, int vz, int r) {
-  PadLayout L;
-  L.b = r + 1;
-  L.px = (((vx + 31) / 32 * 32 + 2 * (r + 1)) + 7) / 8 * 8;
-  L.py = (vy + 31) + 2 * (r + 1) + 4;  // tiles of at most 32 rows, whole quads
-  L.pz = vz + 2 * r + 4;
-  return L;
-}
 
 struct QuadParams {
   FusedParams f;
@@ -36,74 +13,6 @@ struct QuadParams {
   size_t slice, volume;   // strides of the padded images
   int y0;                 // first output row of the launch's tiles
 };
-
-// How the tiles of a group of transforms cover the grid: 24-row tiles, and one
-// row of 16-row tiles below them or none, each in its own launch and z chunks.
-struct QuadPlan {
-  int rows24 = 0, rows16 = 0;  // rows of tiles
-  int z24 = 0, z16 = 0;        // slices per CTA
-  long long cost = 0;          // estimated duration: kQuadW24 per slice of a 24-row tile
-};
-// Times of a slice of a 24- and a 16-row tile: 1.84 and 1.51 us at radius 2,
-// 1.91 and 1.95 at 3 and 4 (the moments threads' serial chain is the same);
-// k_fixed_quad 1.57 and 1.38, 1.41 and 1.41, 1.74 and 1.41.
-constexpr int kQuadW24 = 12, kQuadW16 = 11;
-
-// The plan with the least estimated duration, for one CTA per SM at a time and
-// 2R + 3 slices per CTA beside its output (the windows' run-up, filling and
-// draining). The 1-16 rows that 24-row tiles leave over go to 16-row tiles,
-// which fill the gaps of the 24-row launch's last wave, or, where that gains
-// less than 2 %, to 24-row tiles that reach beyond the grid: one transform at
-// 256^3, radius 4, takes 3 waves of 63 slices either way, and the second launch
-// costs 36 us of 398. Moments against two launches one after the other, the
-// second's chunks chosen by itself: that case 402 -> 362 us, 25 transforms at
-// 135 x 109 x 122, radius 2, 1049 -> 991.
-inline QuadPlan quad_plan(int vx, int vy, int vz, int r, int cnt, int sms, int zchunk) {
-  QuadPlan best;
-  const long long ntx = (vx + 31) / 32, h = 2 * r + 3;
-  sms = sms < 1 ? 1 : sms;
-  // duration of a CTAs of length la, then b of length lb as SMs come free
-  auto duration = [&](long long a, long long la, long long b, long long lb) {
-    const long long part = a % sms, t0 = a / sms * la, t1 = t0 + la;
-    const long long late = b / sms * lb, left = b % sms;  // whole rounds: every SM later by one
-    long long end = (part ? t1 : t0) + late;
-    if (left > sms - part)
-      end = t1 + late + lb;
-    else if (left && t0 + late + lb > end)
-      end = t0 + late + lb;
-    return end;
-  };
-  auto chunks = [&](int zc) { return (vz + zc - 1) / zc; };
-  // chunk sizes to consider for n columns
-  auto try_chunks = [&](long long n, auto f) {
-    if (zchunk > 0) return f(zchunk < vz ? zchunk : vz);
-    for (int nz = 1, last = 0; nz <= vz && nz <= 64 && (nz == 1 || n * nz <= 8LL * sms); ++nz) {
-      const int zc = (vz + nz - 1) / nz;
-      if (zc != last) f(zc);
-      last = zc;
-    }
-  };
-  auto keep = [&](int rows24, int rows16, int z24, int z16, long long cost) {
-    if (!best.z24 || cost < best.cost) best = {rows24, rows16, z24, z16, cost};
-  };
-  const int all24 = (vy + 23) / 24, rest = vy % 24;
-  const long long n24 = ntx * all24 * cnt;
-  try_chunks(n24, [&](int z24) {
-    keep(all24, 0, z24, vz, duration(n24 * chunks(z24), (z24 + h) * kQuadW24, 0, 0));
-  });
-  if (vy > 24 && rest > 0 && rest <= 16) {
-    // a second launch has to save 2 %
-    const long long n = ntx * (vy / 24) * cnt, m = ntx * cnt, bar = best.cost - best.cost / 50;
-    try_chunks(n, [&](int z24) {
-      try_chunks(m, [&](int z16) {
-        const long long d = duration(n * chunks(z24), (z24 + h) * kQuadW24, m * chunks(z16),
-                                     (z16 + h) * kQuadW16);
-        if (d < bar) keep(vy / 24, 1, z24, z16, d);
-      });
-    });
-  }
-  return best;
-}
 
 // The launches of a plan: the second one starts as SMs come free from the first
 // (programmatic dependent launch; both only read what earlier launches wrote
