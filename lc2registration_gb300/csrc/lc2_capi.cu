@@ -184,7 +184,7 @@ struct lc2_context {
   float* d_scratch = nullptr;  // per-slot warped image (+ Sobel when hr_moving)
   int slots = 1;
   size_t per_slot = 0;  // scratch bytes per slot
-  lc2::Xform* d_xf = nullptr;  // cap transforms, and set_fixed's identity
+  lc2::Xform* d_xf = nullptr;
   const lc2::Xform* xf = nullptr;  // what the kernels read: d_xf, or h_xf (direct_call)
   unsigned long long* d_acc = nullptr;
   double* d_out = nullptr;
@@ -193,7 +193,7 @@ struct lc2_context {
   // values: the last kernels of a batch reset what they read, so only new buffers
   // and a launch whose sums were not finalised (another path, an error) are not
   int clean = 0;
-  lc2::Xform* h_xf = nullptr;  // pinned staging, as d_xf
+  lc2::Xform* h_xf = nullptr;  // pinned staging
   double* h_out = nullptr;     // pinned results
   int staged = 0;              // transforms of the last stage or evaluation, in h_xf
   bool xf_stale = false;       // they are not in d_xf (upload_staged)
@@ -204,7 +204,8 @@ struct lc2_context {
   // static ultrasound (HighResolutionModality: Moving): weighting factor per
   // voxel and its exact fixed-point sum
   float* d_sigma = nullptr;
-  int* d_su = nullptr;  // window sum of the quantised static ultrasound per voxel
+  int* d_su = nullptr;  // window sum of the quantised static ultrasound per voxel;
+                        // behind d_sigma in its allocation (static_sums)
   long long sigma_sum = -1;
   // resampled ultrasound (HighResolutionModality: Fixed): the static image
   // and its Sobel quantised, their window sums and centred sums
@@ -267,25 +268,52 @@ struct lc2_context {
 };
 
 namespace lc2 {
+// What a window sum along x reads per voxel: an image; or of the static ultrasound
+// the quantised value, or its square with a mark at bit kInvalidBit for a value
+// <= 1e-6 (cu_lc2_3d.cu:223-243); a window's marks add up above its sum of
+// squares (< 2^50).
+constexpr int kInvalidBit = 52;
+template <typename T>
+struct BoxImage {
+  const T* p;
+  __device__ T operator()(size_t i) const { return p[i]; }
+};
+template <typename TU>
+struct BoxQuant {
+  const TU* u;
+  float qu;
+  __device__ int operator()(size_t i) const { return quant(ldf(u, i), qu); }
+};
+template <typename TU>
+struct BoxSquare {
+  const TU* u;
+  float qu;
+  __device__ long long operator()(size_t i) const {
+    const float v = ldf(u, i);
+    const long long q = quant(v, qu);
+    return q * q + (v > 1e-6f ? 0ll : 1ll << kInvalidBit);
+  }
+};
+
 // Exact window sums of width 2r+1 with zero padding (r <= 12). Bound by their
 // one read and one write of the image. Along x: a warp per row, its values
 // staged in shared memory 128 at a time, each lane summing the windows of four
 // interleaved columns (a running sum per lane would read with a stride).
-template <typename T>
-__global__ void __launch_bounds__(256) k_box_x(const T* __restrict__ in, T* __restrict__ out,
-                                               int nx, long long rows, int r) {
+template <typename T, typename In>
+__global__ void __launch_bounds__(256) k_box_x(In in, T* __restrict__ out, int nx, long long rows,
+                                               int r) {
   __shared__ T s_v[8][128 + 24];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * 8 + w;
   if (row >= rows) return;
-  const T* src = in + row * nx;
-  T* dst = out + row * nx;
+  const size_t first = (size_t)row * nx;
+  T* dst = out + first;
   T* v = s_v[w];
   for (int x0 = 0; x0 < nx; x0 += 128) {
     __syncwarp();
     for (int i = lane; i < 128 + 2 * r; i += 32) {
       const int x = x0 - r + i;
-      v[i] = (x >= 0 && x < nx) ? src[x] : T(0);
+      v[i] = (x >= 0 && x < nx) ? in(first + x) : T(0);
     }
     __syncwarp();
 #pragma unroll
@@ -325,58 +353,54 @@ __global__ void __launch_bounds__(256) k_box_line(const T* __restrict__ in, T* _
   }
 }
 
-// Static ultrasound: quantised values, and their squares with a mark at bit
-// kInvalidBit for a value <= 1e-6 (cu_lc2_3d.cu:223-243); a window's marks add
-// up above its sum of squares (< 2^50).
-constexpr int kInvalidBit = 52;
-template <typename TU>
-__global__ void k_static_u(const TU* __restrict__ U, size_t n, float qu, int* __restrict__ q,
-                           long long* __restrict__ w) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const float u = ldf(U, i);
-    const int v = quant(u, qu);
-    q[i] = v;
-    w[i] = (long long)v * v + (u > 1e-6f ? 0ll : 1ll << kInvalidBit);
-  }
-}
-
-// Weighting factor of every voxel from the window sums S_U and w, as
-// solve_centred computes it (0 where the window leaves the grid, holds an
-// invalid value or has no variance), and the exact sum of all of them.
-__global__ void __launch_bounds__(256) k_sigma(const int* __restrict__ su,
-                                               const long long* __restrict__ w, int nx, int ny,
-                                               int nz, int r, int rz, long long n,
-                                               long long thr_var, float sig_scale, float sum_scale,
-                                               float* __restrict__ sigma,
-                                               unsigned long long* __restrict__ sum) {
-  const size_t nv = (size_t)nx * ny * nz;
+// Weighting factor of every voxel from the window sums S_U and, of w, all but the
+// last axis's (y in 2D, z in 3D), which this sums as k_box_line does: as
+// solve_centred computes it (0 where the window leaves the grid, holds an invalid
+// value or has no variance), and the exact sum of all of them. A line of len
+// voxels `inner` apart at each of the inner positions: along z (deep), of slices
+// of ny rows of nx, or along y.
+__global__ void __launch_bounds__(256) k_sigma_line(const long long* __restrict__ w,
+                                                    const int* __restrict__ su, int nx, int ny,
+                                                    bool deep, int len, int r, long long n,
+                                                    long long thr_var, float sig_scale,
+                                                    float sum_scale, float* __restrict__ sigma,
+                                                    unsigned long long* __restrict__ sum) {
+  const long long inner = deep ? (long long)nx * ny : nx;
+  const long long line = (long long)blockIdx.x * 256 + threadIdx.x;
   long long acc = 0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const size_t l = i / nx;
-    const int x = (int)(i - l * nx), z = (int)(l / ny), y = (int)(l - (size_t)z * ny);
-    float sg = 0.0f;
-    const long long s = su[i], uu = w[i];
-    if (x >= r && x + r < nx && y >= r && y + r < ny && z >= rz && z + rz < nz &&
-        (uu >> kInvalidBit) == 0) {
-      const long long d = n * uu - s * s;
-      if (d > thr_var) sg = sqrtf(ll2f(d)) * sig_scale;
+  if (line < inner) {
+    const int y = (int)(line / nx), x = (int)(line - (long long)y * nx);
+    const bool in = x >= r && x + r < nx && (!deep || (y >= r && y + r < ny));
+    for (int j0 = blockIdx.y * kBoxSeg; j0 < len; j0 += gridDim.y * kBoxSeg) {
+      const int j1 = min(j0 + kBoxSeg, len);
+      long long uu = 0;
+      for (int j = max(j0 - r, 0); j < min(j0 + r, len); ++j) uu += w[line + (size_t)j * inner];
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        const size_t i = line + (size_t)j * inner;
+        if (j + r < len) uu += w[i + (size_t)r * inner];
+        float sg = 0.0f;
+        if (in && j >= r && j + r < len && (uu >> kInvalidBit) == 0) {
+          const long long s = su[i], d = n * uu - s * s;
+          if (d > thr_var) sg = sqrtf(ll2f(d)) * sig_scale;
+        }
+        sigma[i] = sg;
+        acc += __float2int_rn(sg * sum_scale);
+        if (j - r >= 0) uu -= w[i - (size_t)r * inner];
+      }
     }
-    sigma[i] = sg;
-    acc += __float2int_rn(sg * sum_scale);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(sum, (unsigned long long)acc);
 }
 
 // An image of rows nx and ny rows per slice into padded strides.
-__global__ void k_pad(const int* __restrict__ in, int nx, int ny, size_t n, int* __restrict__ out,
-                      int row, size_t plane) {
+template <typename In>
+__global__ void k_pad(In in, int nx, int ny, size_t n, int* __restrict__ out, int row, size_t plane) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const size_t l = i / nx, z = l / ny;
-    out[z * plane + (l - z * ny) * row + (i - l * nx)] = in[i];
+    out[z * plane + (l - z * ny) * row + (i - l * nx)] = in(i);
   }
 }
 
@@ -569,12 +593,12 @@ int ensure_capacity(lc2_context* c, int count) {
   c->d_xf = nullptr; c->d_acc = nullptr; c->d_out = nullptr; c->h_xf = nullptr; c->h_out = nullptr;
   c->cap = 0;
   c->staged = 0;
-  LC2_CUDA(dev_alloc((void**)&c->d_xf, sizeof(lc2::Xform) * (ncap + 1), c->stream));
+  LC2_CUDA(dev_alloc((void**)&c->d_xf, sizeof(lc2::Xform) * ncap, c->stream));
   c->xf = c->d_xf;
   LC2_CUDA(dev_alloc((void**)&c->d_acc, sizeof(unsigned long long) * 2 * ncap, c->stream));
   c->clean = 0;
   LC2_CUDA(dev_alloc((void**)&c->d_out, sizeof(double) * ncap, c->stream));
-  LC2_CUDA(host_alloc((void**)&c->h_xf, sizeof(lc2::Xform) * (ncap + 1)));
+  LC2_CUDA(host_alloc((void**)&c->h_xf, sizeof(lc2::Xform) * ncap));
   LC2_CUDA(host_alloc((void**)&c->h_out, sizeof(double) * ncap));
   if (c->mi) {
     dev_free(c->d_hist, c->stream);
@@ -1246,17 +1270,17 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
     h += c->nv * (4 * sizeof(int) + 3 * sizeof(long long) + sizeof(float4));
   if (c->mi)
     h += c->nv + 64 * (sizeof(unsigned) * (lc2::kMiHist + 2) + sizeof(double) * 2 * lc2::kMiParts);
-  h += sizeof(lc2::Xform) + 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
+  h += 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
+  h += sizeof(int);  // d_err
   if (c->presample)  // the presample buffer at its largest
     h += sizeof(float) * std::max(presample_voxels(c, c->quad) * (size_t)presample_cap(c, c->quad),
                                   c->nv * (size_t)presample_cap(c, false));
   // padded static fields: quantised ultrasound and its (sigma, S_U), or M and G
   if (c->quad) h += (hrm ? sizeof(int) + sizeof(int2) : 2 * sizeof(int)) * c->lay.volume();
   *held = h;
-  // both images, and the temporaries of the static sums
-  *peak_extra = (c->nm + c->nf) * sizeof(float);
-  if (!c->mi)
-    *peak_extra += c->nv * (hrm ? 2 * sizeof(long long) : 2 * sizeof(int) + sizeof(long long));
+  // one image at a time, then the temporary of the Fixed static sums
+  *peak_extra = std::max(c->nm, c->nf) * sizeof(float);
+  if (!hrm && !c->mi) *peak_extra = std::max(*peak_extra, c->nv * sizeof(long long));
 }
 
 int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
@@ -1288,9 +1312,8 @@ int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
   if (e == cudaSuccess && !cfg->high_res_is_moving)
     e = dev_alloc((void**)&c->d_gstatic, c->nv * sizeof(float), c->stream);
   if (e == cudaSuccess && cfg->high_res_is_moving && !c->mi)
-    e = dev_alloc((void**)&c->d_sigma, c->nv * sizeof(float), c->stream);
-  if (e == cudaSuccess && cfg->high_res_is_moving && !c->mi)
-    e = dev_alloc((void**)&c->d_su, c->nv * sizeof(int), c->stream);
+    e = dev_alloc((void**)&c->d_sigma, c->nv * (sizeof(float) + sizeof(int)), c->stream);
+  if (e == cudaSuccess && c->d_sigma) c->d_su = reinterpret_cast<int*>(c->d_sigma + c->nv);
   if (e == cudaSuccess && c->quad)
     e = dev_alloc((void**)&c->d_uq,
                   c->lay.volume() * (cfg->high_res_is_moving ? 1 : 2) * sizeof(int), c->stream);
@@ -1357,7 +1380,6 @@ int lc2_destroy(lc2_context* c) {
   dev_free(c->d_static, fs);
   dev_free(c->d_gstatic, fs);
   dev_free(c->d_sigma, fs);
-  dev_free(c->d_su, fs);
   dev_free(c->d_pre, fs);
   dev_free(c->d_uq, fs);
   dev_free(c->d_ss, fs);
@@ -1573,18 +1595,26 @@ __global__ void __launch_bounds__(256) k_absmax_flag(const float* __restrict__ a
   }
 }
 
-// Largest |value| of n device floats; *bad: NaN/Inf among them. For two images.
-int device_absmax(lc2_context* c, const float* a, size_t na, const float* b, size_t nb, float mx[2],
-                  bool bad[2]) {
-  unsigned int* flags = reinterpret_cast<unsigned int*>(c->d_acc);  // 4 words, reset below
-  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
-  const int blocks = 152 * 6;
-  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(a, na, flags);
-  k_absmax_flag<<<blocks, 256, 0, c->stream>>>(b, nb, flags + 2);
+// Largest |value| of two device images, and whether NaN/Inf are among them: an
+// image's words are cleared for both and filled by absmax_launch, in any order
+// with other work of the stream, and read by absmax_read.
+unsigned int* absmax_words(lc2_context* c) { return reinterpret_cast<unsigned int*>(c->d_acc); }
+
+int absmax_clear(lc2_context* c) {
+  if (!c->mi) c->clean = 0;
+  LC2_CUDA(cudaMemsetAsync(absmax_words(c), 0, 4 * sizeof(unsigned int), c->stream));
+  return LC2_OK;
+}
+
+int absmax_launch(lc2_context* c, const float* a, size_t n, int image) {
+  k_absmax_flag<<<152 * 6, 256, 0, c->stream>>>(a, n, absmax_words(c) + 2 * image);
   LC2_CUDA(cudaGetLastError());
+  return LC2_OK;
+}
+
+int absmax_read(lc2_context* c, float mx[2], bool bad[2]) {
   unsigned int h[4] = {0, 0, 0, 0};
-  LC2_CUDA(cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  LC2_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), c->stream));
+  LC2_CUDA(cudaMemcpyAsync(h, absmax_words(c), sizeof(h), cudaMemcpyDeviceToHost, c->stream));
   LC2_CUDA(cudaStreamSynchronize(c->stream));
   for (int i = 0; i < 2; ++i) {
     std::memcpy(&mx[i], &h[2 * i], 4);
@@ -1602,83 +1632,87 @@ struct TempBuffer {
     st = s;
     return dev_alloc((void**)&p, n * sizeof(T), s);
   }
-  ~TempBuffer() { dev_free(p, st); }
+  void free() {
+    dev_free(p, st);
+    p = nullptr;
+  }
+  ~TempBuffer() { free(); }
 };
 
-// Window sums over the context's patch of the image in a, into out or, without
-// one, into b (3D) or a (2D); returns where. a and b are overwritten; a pass
-// never writes what it reads.
-template <typename T>
-T* box_sums(lc2_context* c, T* a, T* b, T* out = nullptr) {
-  const long long nx = c->virt.dim[0], ny = c->virt.dim[1], nz = c->virt.dim[2];
-  const int r = c->cfg.patch_size;
-  auto line = [&](const T* src, T* dst, long long inner, long long outer, size_t stride, size_t group,
-                  long long len) {
-    dim3 grid((unsigned)((inner * outer + 255) / 256),
-              (unsigned)std::min<long long>((len + lc2::kBoxSeg - 1) / lc2::kBoxSeg, 65535));
-    lc2::k_box_line<T><<<grid, 256, 0, c->stream>>>(src, dst, inner, outer, stride, group, (int)len, r);
-    ++c->launches;
-  };
-  lc2::k_box_x<T><<<(unsigned)((ny * nz + 7) / 8), 256, 0, c->stream>>>(a, b, (int)nx, ny * nz, r);
+// The passes of window sums over the context's patch, out of place: along x from
+// any source, along y, along z.
+template <typename T, typename In>
+void box_x(lc2_context* c, In in, T* out) {
+  const long long rows = (long long)c->virt.dim[1] * c->virt.dim[2];
+  lc2::k_box_x<T, In><<<(unsigned)((rows + 7) / 8), 256, 0, c->stream>>>(in, out, c->virt.dim[0], rows,
+                                                                         c->cfg.patch_size);
   ++c->launches;
-  if (c->lc2_nd == 2) {
-    if (!out) out = a;
-    line(b, out, nx, nz, (size_t)nx, (size_t)(nx * ny), ny);
-    return out;
-  }
-  line(b, a, nx, nz, (size_t)nx, (size_t)(nx * ny), ny);
-  if (!out) out = b;
-  line(a, out, nx * ny, 1, (size_t)(nx * ny), 0, nz);
-  return out;
+}
+dim3 box_grid(long long lines, int len) {
+  return dim3((unsigned)((lines + 255) / 256),
+              (unsigned)std::min((len + lc2::kBoxSeg - 1) / lc2::kBoxSeg, 65535));
+}
+template <typename T>
+void box_y(lc2_context* c, const T* in, T* out) {
+  const long long nx = c->virt.dim[0], ny = c->virt.dim[1], nz = c->virt.dim[2];
+  lc2::k_box_line<T><<<box_grid(nx * nz, (int)ny), 256, 0, c->stream>>>(
+      in, out, nx, nz, (size_t)nx, (size_t)(nx * ny), (int)ny, c->cfg.patch_size);
+  ++c->launches;
+}
+template <typename T>
+void box_z(lc2_context* c, const T* in, T* out) {
+  const long long slice = (long long)c->virt.dim[0] * c->virt.dim[1];
+  const int nz = c->virt.dim[2];
+  lc2::k_box_line<T><<<box_grid(slice, nz), 256, 0, c->stream>>>(in, out, slice, 1, (size_t)slice, 0,
+                                                                 nz, c->cfg.patch_size);
+  ++c->launches;
 }
 
 // Static ultrasound: its window sums S_U, weighting factors and their sum, by
-// exact box sums. With it, the checks on the device and the fixed image through
-// k_presample, lc2_set_images takes 24.5 -> 1.6 ms on 256^3 host volumes and
-// 2.3 -> 0.29 ms for 128^3 -> 96^3 (the generic moments kernel alone took 1.4,
-// line-by-line sums 0.4 and the host's scan for NaN about 20 ms).
-int static_sums(lc2_context* c) {
-  const lc2_geometry& v = c->virt;
+// exact box sums in the buffers the context holds: scratch slot 0 and d_sigma
+// with d_su behind it are eight bytes per voxel each. With it, the checks on the
+// device and the fixed image through k_presample, lc2_set_images takes 24.5 ->
+// 1.6 ms on 256^3 host volumes and 2.3 -> 0.29 ms for 128^3 -> 96^3 (the generic
+// moments kernel alone took 1.4, line-by-line sums 0.4 and the host's scan for
+// NaN about 20 ms).
+template <typename TU>
+int static_sums(lc2_context* c, const TU* u) {
   const size_t nv = c->nv;
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
-  const int st = c->cfg.storage;
-  const int nx = v.dim[0], ny = v.dim[1], nz = v.dim[2], r = c->cfg.patch_size;
-  int* q = reinterpret_cast<int*>(c->d_scratch);
-  int* tq = q + nv;  // the slot holds two planes of nv floats
-  TempBuffer<long long> w, tw;
-  LC2_CUDA(w.alloc(nv, c->stream));
-  LC2_CUDA(tw.alloc(nv, c->stream));
-  auto with_u = [&](auto* u) {
-    lc2::k_static_u<<<blocks, 256, 0, c->stream>>>(u, nv, c->fp.qu, q, w.p);
-  };
-  if (st == LC2_STORE_F16)
-    with_u((const __half*)c->d_static);
-  else if (st == LC2_STORE_BF16)
-    with_u((const __nv_bfloat16*)c->d_static);
-  else
-    with_u((const float*)c->d_static);
-  ++c->launches;
-  if (c->quad) {
-    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.volume() * sizeof(int), c->stream));
-    LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.volume() * sizeof(int2), c->stream));
-    lc2::k_pad<<<blocks, 256, 0, c->stream>>>(q, nx, ny, nv,
-                                              c->d_uq + c->lay.first() + c->lay.origin(), c->lay.px,
-                                              c->lay.slice());
-    ++c->launches;
+  const int nx = c->virt.dim[0], ny = c->virt.dim[1], nz = c->virt.dim[2];
+  const lc2::BoxQuant<TU> quantised{u, c->fp.qu};
+  const lc2::BoxSquare<TU> square{u, c->fp.qu};
+  long long* w = reinterpret_cast<long long*>(c->d_scratch);
+  int* tmp = reinterpret_cast<int*>(c->d_sigma);
+  if (c->lc2_nd == 3) {
+    long long* both = reinterpret_cast<long long*>(c->d_sigma);
+    box_x(c, square, both);
+    box_y(c, both, w);
+    box_x(c, quantised, c->d_su);
+    box_y(c, c->d_su, tmp);
+    box_z(c, tmp, c->d_su);
+  } else {
+    box_x(c, square, w);
+    box_x(c, quantised, tmp);
+    box_y(c, tmp, c->d_su);
   }
-  box_sums(c, q, tq, c->d_su);
-  const long long* sums = box_sums(c, w.p, tw.p);
   c->clean = 0;
   LC2_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long), c->stream));
-  lc2::k_sigma<<<blocks, 256, 0, c->stream>>>(c->d_su, sums, nx, ny, nz, r, c->lc2_nd == 3 ? r : 0,
-                                              (long long)c->n, c->mp.thr_var, c->mp.sig_scale,
-                                              c->mp.sum_scale, c->d_sigma, c->d_acc);
+  const bool deep = c->lc2_nd == 3;
+  const int len = deep ? nz : ny;
+  lc2::k_sigma_line<<<box_grid(deep ? (long long)nx * ny : nx, len), 256, 0, c->stream>>>(
+      w, c->d_su, nx, ny, deep, len, c->cfg.patch_size, (long long)c->n, c->mp.thr_var,
+      c->mp.sig_scale, c->mp.sum_scale, c->d_sigma, c->d_acc);
   ++c->launches;
   if (c->quad) {
-    lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(
-        c->d_sigma, c->d_su, nx, ny, nv, c->d_ss + c->lay.first() + c->lay.origin(), c->lay.px,
-        c->lay.slice());
-    ++c->launches;
+    const size_t first = c->lay.first() + c->lay.origin();
+    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.volume() * sizeof(int), c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.volume() * sizeof(int2), c->stream));
+    lc2::k_pad<<<blocks, 256, 0, c->stream>>>(quantised, nx, ny, nv, c->d_uq + first, c->lay.px,
+                                              c->lay.slice());
+    lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(c->d_sigma, c->d_su, nx, ny, nv, c->d_ss + first,
+                                                     c->lay.px, c->lay.slice());
+    c->launches += 2;
   }
   LC2_CUDA(cudaGetLastError());
   unsigned long long sum = 0;
@@ -1695,11 +1729,10 @@ int fixed_static_sums(lc2_context* c) {
   const lc2_geometry& v = c->virt;
   const size_t nv = c->nv;
   const int nx = v.dim[0], ny = v.dim[1];
-  TempBuffer<int> ti, tj;
   TempBuffer<long long> tl;
-  LC2_CUDA(ti.alloc(nv, c->stream));
-  LC2_CUDA(tj.alloc(nv, c->stream));
   LC2_CUDA(tl.alloc(nv, c->stream));
+  int* ti = reinterpret_cast<int*>(tl.p);
+  int* tj = reinterpret_cast<int*>(c->d_scratch);  // slot 0
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 16);
   lc2::k_fixed_quant<<<blocks, 256, 0, c->stream>>>((const float*)c->d_static, c->d_gstatic, nv,
                                                     c->fp.qm, c->fp.qg, c->d_fq, c->d_fd);
@@ -1707,21 +1740,27 @@ int fixed_static_sums(lc2_context* c) {
     LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, 2 * c->lay.volume() * sizeof(int), c->stream));
     for (int f = 0; f < 2; ++f)
       lc2::k_pad<<<blocks, 256, 0, c->stream>>>(
-          c->d_fq + f * nv, nx, ny, nv,
+          lc2::BoxImage<int>{c->d_fq + f * nv}, nx, ny, nv,
           c->d_uq + f * c->lay.volume() + c->lay.first() + c->lay.origin(), c->lay.px,
           c->lay.slice());
     c->launches += 2;
   }
-  // S_M, S_G (from a copy of q, which stays), then S_MM, S_GG, S_MG in place in d
+  // S_M, S_G, then S_MM, S_GG, S_MG in place in d
+  const bool deep = c->lc2_nd == 3;
   for (int f = 0; f < 2; ++f) {
-    LC2_CUDA(cudaMemcpyAsync(ti.p, c->d_fq + f * nv, nv * sizeof(int), cudaMemcpyDeviceToDevice,
-                             c->stream));
-    box_sums(c, ti.p, tj.p, c->d_fs + f * nv);
+    int* sums = c->d_fs + f * nv;
+    box_x(c, lc2::BoxImage<int>{c->d_fq + f * nv}, ti);
+    box_y(c, ti, deep ? tj : sums);
+    if (deep) box_z(c, tj, sums);
   }
   for (int f = 0; f < 3; ++f) {
     long long* d = c->d_fd + f * nv;
-    if (box_sums(c, d, tl.p) != d)
+    box_x(c, lc2::BoxImage<long long>{d}, tl.p);
+    box_y(c, tl.p, d);
+    if (deep) {
+      box_z(c, d, tl.p);
       LC2_CUDA(cudaMemcpyAsync(d, tl.p, nv * sizeof(long long), cudaMemcpyDeviceToDevice, c->stream));
+    }
   }
   lc2::k_fixed_centre<<<blocks, 256, 0, c->stream>>>(c->d_fs, c->d_fd, nv, (long long)c->n);
   // the solve factors, and (S_M, S_G) interleaved per voxel through the
@@ -1744,18 +1783,20 @@ int set_static_bins(lc2_context* c) {
   const int ustore = c->cfg.high_res_is_moving ? c->cfg.storage : LC2_STORE_F32;
   float* img = c->d_scratch;  // slot 0
   LC2_TRY(to_float(c, c->d_static, img, nv, ustore));
-  TempBuffer<unsigned long long> t;  // counts, then the range's two words
-  LC2_CUDA(t.alloc(lc2::kMiBins + 1, c->stream));
-  unsigned* range = reinterpret_cast<unsigned*>(t.p + lc2::kMiBins);
-  LC2_CUDA(cudaMemsetAsync(t.p, 0, (lc2::kMiBins + 1) * sizeof(unsigned long long), c->stream));
+  // counts, then the range's two words, in the first histogram, zeroed again below
+  unsigned long long* t = reinterpret_cast<unsigned long long*>(c->d_hist);
+  const size_t bytes = (lc2::kMiBins + 1) * sizeof(unsigned long long);
+  unsigned* range = reinterpret_cast<unsigned*>(t + lc2::kMiBins);
+  LC2_CUDA(cudaMemsetAsync(t, 0, bytes, c->stream));
   LC2_CUDA(cudaMemsetAsync(range, 0xff, sizeof(unsigned), c->stream));
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 152 * 8);
   lc2::k_mi_static_range<><<<blocks, 256, 0, c->stream>>>(img, nv, range);
-  lc2::k_mi_static_bins<><<<blocks, 256, 0, c->stream>>>(img, nv, range, c->d_sbin, t.p);
+  lc2::k_mi_static_bins<><<<blocks, 256, 0, c->stream>>>(img, nv, range, c->d_sbin, t);
   c->launches += 2;
   LC2_CUDA(cudaGetLastError());
   unsigned long long counts[lc2::kMiBins];
-  LC2_CUDA(cudaMemcpyAsync(counts, t.p, sizeof(counts), cudaMemcpyDeviceToHost, c->stream));
+  LC2_CUDA(cudaMemcpyAsync(counts, t, sizeof(counts), cudaMemcpyDeviceToHost, c->stream));
+  LC2_CUDA(cudaMemsetAsync(t, 0, bytes, c->stream));
   LC2_CUDA(cudaStreamSynchronize(c->stream));
   double s = 0.0;
   for (unsigned long long n : counts)
@@ -1765,25 +1806,21 @@ int set_static_bins(lc2_context* c) {
   return LC2_OK;
 }
 
-// Everything that depends on the fixed image (device floats), given both
-// images' largest |value|: the fixed image on the virtual grid, the fixed-point
-// parameters and the static fields.
-int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
-  const int storage = c->cfg.storage;
-  drop_graphs(c);  // they hold the old images' fixed-point scales
-  // fixed volume resampled onto the virtual grid through the identity
-  // (VirtualToFixed, src/Interpolator/interpolator.cu:526-528)
+// The fixed image (device floats) resampled onto the virtual grid through the
+// identity (VirtualToFixed, src/Interpolator/interpolator.cu:526-528), into
+// scratch slot 0.
+int sample_fixed(lc2_context* c, const float* fixed) {
   lc2::Xform id{};
   {
     float ident[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
     float ident2[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
     build_xform(c->warp_nd, c->virt, c->cfg.fixed, c->warp_nd == 2 ? ident2 : ident, &id);
   }
-  c->h_xf[c->cap] = id;  // behind the staged transforms, which stay
-  const lc2::Xform* d_id = c->d_xf + c->cap;
-  LC2_CUDA(cudaMemcpyAsync(c->d_xf + c->cap, c->h_xf + c->cap, sizeof(lc2::Xform),
-                           cudaMemcpyHostToDevice, c->stream));
-  float* vfix = c->d_scratch;  // slot 0 as temporary
+  // behind absmax_words; the staged transforms in d_xf stay
+  lc2::Xform* d_id = reinterpret_cast<lc2::Xform*>(c->d_acc + 2);
+  if (!c->mi) c->clean = 0;
+  LC2_CUDA(cudaMemcpyAsync(d_id, &id, sizeof(id), cudaMemcpyHostToDevice, c->stream));
+  float* vfix = c->d_scratch;
   if (c->warp_nd == 3) {
     // k_presample's samples are launch_warp's (145 us at 256^3), four times as fast
     lc2::FusedParams S{};
@@ -1793,12 +1830,21 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
     S.vx = c->virt.dim[0];
     S.vy = c->virt.dim[1];
     S.vz = c->virt.dim[2];
-    LC2_CUDA(lc2::presample_launch<float>(fixed, S, d_id, 0, 1, vfix, S.vx,
-                                          (size_t)S.vx * S.vy, c->nv, c->stream));
+    LC2_CUDA(lc2::presample_launch<float>(fixed, S, d_id, 0, 1, vfix, S.vx, (size_t)S.vx * S.vy,
+                                          c->nv, c->stream));
     ++c->launches;
-  } else {
-    LC2_TRY(launch_warp(c, 2, fixed, LC2_STORE_F32, c->cfg.fixed, d_id, 0, 1, vfix, c->nv));
+    return LC2_OK;
   }
+  return launch_warp(c, 2, fixed, LC2_STORE_F32, c->cfg.fixed, d_id, 0, 1, vfix, c->nv);
+}
+
+// Everything that depends on the fixed image sampled by sample_fixed, given both
+// images' largest |value|: the static image, the fixed-point parameters and the
+// static fields.
+int set_fixed(lc2_context* c, float fmax, float mmax) {
+  const int storage = c->cfg.storage;
+  drop_graphs(c);  // they hold the old images' fixed-point scales
+  const float* vfix = c->d_scratch;
   if (c->cfg.high_res_is_moving) {
     LC2_TRY(convert_to_storage(c, vfix, c->d_static, c->nv, storage));
   } else {
@@ -1855,11 +1901,14 @@ int set_fixed(lc2_context* c, const float* fixed, float fmax, float mmax) {
   // limb split: every low limb's window sum (n+1 terms) stays below 2^30
   F.kbits = 0;
   while (((long long)(c->n + 1) << (F.kbits + 1)) <= (1LL << 30)) ++F.kbits;
-  if (c->cfg.high_res_is_moving) {
-    LC2_TRY(static_sums(c));
-  } else {
+  if (!c->cfg.high_res_is_moving)
     LC2_TRY(fixed_static_sums(c));
-  }
+  else if (storage == LC2_STORE_F16)
+    LC2_TRY(static_sums(c, (const __half*)c->d_static));
+  else if (storage == LC2_STORE_BF16)
+    LC2_TRY(static_sums(c, (const __nv_bfloat16*)c->d_static));
+  else
+    LC2_TRY(static_sums(c, (const float*)c->d_static));
   c->ready = true;
   return LC2_OK;
 }
@@ -1874,20 +1923,29 @@ int lc2_set_images(lc2_context* c, const float* fixed, const float* moving) {
   if (!c->owns_moving)
     return fail(LC2_ERR_INVALID_ARGUMENT, "the frames of a stack share the stack's moving volume");
   LC2_TRY(select_device(c));
-  // both images to the device, where they are checked
-  TempBuffer<float> f, m;
-  LC2_CUDA(f.alloc(c->nf, c->stream));
-  LC2_CUDA(m.alloc(c->nm, c->stream));
-  LC2_CUDA(cudaMemcpyAsync(f.p, fixed, sizeof(float) * c->nf, cudaMemcpyHostToDevice, c->stream));
-  LC2_CUDA(cudaMemcpyAsync(m.p, moving, sizeof(float) * c->nm, cudaMemcpyHostToDevice, c->stream));
+  // one image at a time to the device, where it is checked; the context's own
+  // images stay until both are found good
   float mx[2];
   bool bad[2];
-  LC2_TRY(device_absmax(c, f.p, c->nf, m.p, c->nm, mx, bad));
+  LC2_TRY(absmax_clear(c));
+  {
+    TempBuffer<float> f;
+    LC2_CUDA(f.alloc(c->nf, c->stream));
+    LC2_CUDA(cudaMemcpyAsync(f.p, fixed, sizeof(float) * c->nf, cudaMemcpyHostToDevice, c->stream));
+    LC2_TRY(absmax_launch(c, f.p, c->nf, 0));
+    LC2_TRY(sample_fixed(c, f.p));
+  }
+  TempBuffer<float> m;
+  LC2_CUDA(m.alloc(c->nm, c->stream));
+  LC2_CUDA(cudaMemcpyAsync(m.p, moving, sizeof(float) * c->nm, cudaMemcpyHostToDevice, c->stream));
+  LC2_TRY(absmax_launch(c, m.p, c->nm, 1));
+  LC2_TRY(absmax_read(c, mx, bad));
   if (bad[0]) LC2_TRY(image_absmax(fixed, c->nf, "fixed", &mx[0]));  // names the first
   if (bad[1]) LC2_TRY(image_absmax(moving, c->nm, "moving", &mx[1]));
   c->ready = false;
   LC2_TRY(convert_to_storage(c, m.p, c->d_moving, c->nm, c->cfg.storage));
-  return set_fixed(c, f.p, mx[0], mx[1]);
+  m.free();
+  return set_fixed(c, mx[0], mx[1]);
 }
 
 int lc2_set_images_device(lc2_context* c, const float* fixed, const float* moving) {
@@ -1908,12 +1966,16 @@ int lc2_set_images_device(lc2_context* c, const float* fixed, const float* movin
   }
   float mx[2];
   bool bad[2];
-  LC2_TRY(device_absmax(c, fixed, c->nf, moving, c->nm, mx, bad));
+  LC2_TRY(absmax_clear(c));
+  LC2_TRY(absmax_launch(c, fixed, c->nf, 0));
+  LC2_TRY(absmax_launch(c, moving, c->nm, 1));
+  LC2_TRY(absmax_read(c, mx, bad));
   if (bad[0]) return fail(LC2_ERR_INVALID_ARGUMENT, "fixed image has NaN/Inf");
   if (bad[1]) return fail(LC2_ERR_INVALID_ARGUMENT, "moving image has NaN/Inf");
   c->ready = false;
+  LC2_TRY(sample_fixed(c, fixed));
   LC2_TRY(convert_to_storage(c, moving, c->d_moving, c->nm, c->cfg.storage));
-  return set_fixed(c, fixed, mx[0], mx[1]);
+  return set_fixed(c, mx[0], mx[1]);
 }
 
 }  // extern "C"
@@ -2561,9 +2623,11 @@ int lc2_stack_add_frame(lc2_stack* s, const lc2_geometry* frame, const float vir
     cudaError_t e = u.alloc(c->nf, c->stream);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(u.p, ultrasound, sizeof(float) * c->nf, cudaMemcpyHostToDevice, c->stream);
-    st = e == cudaSuccess ? set_fixed(c, u.p, fmax, s->mmax)
+    st = e == cudaSuccess ? sample_fixed(c, u.p)
                           : fail(e == cudaErrorMemoryAllocation ? LC2_ERR_OUT_OF_MEMORY : LC2_ERR_CUDA,
                                  "frame upload: %s", cudaGetErrorString(e));
+    u.free();
+    if (st == LC2_OK) st = set_fixed(c, fmax, s->mmax);
   }
   if (st != LC2_OK) {
     std::string msg = g_err;
