@@ -200,7 +200,7 @@ enum { LC2_OPTION_GENERIC = 7 };
 /* LC2_OPTION_PRESAMPLE (3D, HighResolutionModality Moving): how the moving
  * image is resampled. 1 (the default of such contexts): in a pass of its own,
  * one float per virtual voxel and transform written to a context buffer that
- * grows with the batch up to 2 GiB (26 transforms at 256^3; larger batches
+ * grows with the batch up to 2 GiB (25 transforms at 256^3; larger batches
  * run in groups), which the fused kernel then reads; 0: inside the fused
  * kernel. Other values are refused (LC2_ERR_INVALID_ARGUMENT). Each voxel is
  * sampled once from its 32 x 8 tile's base in form 1 and from the fused

@@ -791,12 +791,14 @@ int tile_rows(const lc2_context* c) {
   return (c->cfg.high_res_is_moving && r >= 3) ? 24 : 16;
 }
 
-// The fused kernel (static ultrasound): one launch for `cnt` transforms.
-// The presample buffer holds the images of a group of transforms, at most
-// 2 GiB and 64 transforms -- 26 padded ones at 256^3. It grows with the batches a context is
-// given (a registration's single evaluations hold one slot); growing moves
-// it, which drops the captured graphs that name it.
-constexpr size_t kPresampleBytes = size_t(2) << 30;
+// The presample buffer holds the images of a group of transforms. It grows with
+// the batches a context is given (a registration's single evaluations hold one
+// slot); growing moves it, which drops the captured graphs that name it. It and
+// the quad kernels' static fields together take 64 images of the grid's voxels
+// at most, no more than 2 GiB of them (25 padded ones at 256^3), but never less
+// than one slot, and 32 MiB where 64 images are less: groups of small grids
+// should fill the device.
+constexpr size_t kPresampleBytes = size_t(2) << 30, kPresampleSmall = size_t(32) << 20;
 
 // Whether the context's batches run on k_fused_quad or k_fixed_quad: presampled
 // images at radius <= 4, unless 8- or 16-row tiles are asked for.
@@ -805,14 +807,27 @@ bool use_quad(const lc2_context* c) {
          tile_rows(c) == 24;
 }
 
-// Voxels of one presampled image in the layout in use.
-size_t presample_voxels(const lc2_context* c, bool padded) {
-  return padded ? c->lay.volume() : c->nv;
+// Bytes of n presampled images in a layout.
+size_t presample_bytes(const lc2_context* c, bool padded, int n) {
+  return sizeof(float) * (padded ? c->lay.total(n) : c->nv * (size_t)n);
+}
+
+// Bytes of the padded static fields: quantised ultrasound and its (sigma, S_U),
+// or M and G.
+size_t quad_field_bytes(const lc2_context* c) {
+  if (!c->quad) return 0;
+  if (c->cfg.high_res_is_moving) return c->lay.total(1) * (sizeof(int) + sizeof(int2));
+  return c->lay.total(2) * sizeof(int);
 }
 
 int presample_cap(const lc2_context* c, bool padded) {
-  const size_t per = sizeof(float) * presample_voxels(c, padded);
-  return (int)std::max<size_t>(1, std::min<size_t>(64, kPresampleBytes / per));
+  const size_t image = sizeof(float) * c->nv;
+  size_t most = image * std::max<size_t>(1, std::min<size_t>(64, kPresampleBytes / image));
+  if (c->quad) most = std::max(most, kPresampleSmall);
+  const size_t fields = quad_field_bytes(c);
+  int n = 1;
+  while (n < 64 && fields + presample_bytes(c, padded, n + 1) <= most) ++n;
+  return n;
 }
 
 // The padded layout's borders are zeroed once, here: k_presample writes the
@@ -825,7 +840,7 @@ int ensure_presample(lc2_context* c, int count) {
   dev_free(c->d_pre, c->stream);
   c->d_pre = nullptr;
   c->pre_slots = 0;
-  const size_t bytes = sizeof(float) * presample_voxels(c, padded) * (size_t)want;
+  const size_t bytes = presample_bytes(c, padded, want);
   LC2_CUDA(dev_alloc((void**)&c->d_pre, bytes, c->stream));
   if (padded) LC2_CUDA(cudaMemsetAsync(c->d_pre, 0, bytes, c->stream));
   c->pre_slots = want;
@@ -838,7 +853,7 @@ int launch_presample(lc2_context* c, int k0, int n) {
   const bool padded = c->pre_padded;
   const int row = padded ? c->lay.px : c->virt.dim[0];
   const size_t plane = padded ? c->lay.slice() : (size_t)c->virt.dim[0] * c->virt.dim[1];
-  const size_t volume = presample_voxels(c, padded);
+  const size_t volume = padded ? c->lay.volume() : c->nv;
   float* out = c->d_pre + (padded ? c->lay.first() + c->lay.origin() : 0);
   TimerScope ts(c, K_WARP);
   cudaError_t e;
@@ -1273,10 +1288,9 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
   h += 64 * (sizeof(lc2::Xform) + 2 * sizeof(unsigned long long) + sizeof(double));
   h += sizeof(int);  // d_err
   if (c->presample)  // the presample buffer at its largest
-    h += sizeof(float) * std::max(presample_voxels(c, c->quad) * (size_t)presample_cap(c, c->quad),
-                                  c->nv * (size_t)presample_cap(c, false));
-  // padded static fields: quantised ultrasound and its (sigma, S_U), or M and G
-  if (c->quad) h += (hrm ? sizeof(int) + sizeof(int2) : 2 * sizeof(int)) * c->lay.volume();
+    h += std::max(presample_bytes(c, c->quad, presample_cap(c, c->quad)),
+                  presample_bytes(c, false, presample_cap(c, false)));
+  h += quad_field_bytes(c);
   *held = h;
   // one image at a time, then the temporary of the Fixed static sums
   *peak_extra = std::max(c->nm, c->nf) * sizeof(float);
@@ -1315,10 +1329,10 @@ int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
     e = dev_alloc((void**)&c->d_sigma, c->nv * (sizeof(float) + sizeof(int)), c->stream);
   if (e == cudaSuccess && c->d_sigma) c->d_su = reinterpret_cast<int*>(c->d_sigma + c->nv);
   if (e == cudaSuccess && c->quad)
-    e = dev_alloc((void**)&c->d_uq,
-                  c->lay.volume() * (cfg->high_res_is_moving ? 1 : 2) * sizeof(int), c->stream);
+    e = dev_alloc((void**)&c->d_uq, c->lay.total(cfg->high_res_is_moving ? 1 : 2) * sizeof(int),
+                  c->stream);
   if (e == cudaSuccess && c->quad && cfg->high_res_is_moving)
-    e = dev_alloc((void**)&c->d_ss, c->lay.volume() * sizeof(int2), c->stream);
+    e = dev_alloc((void**)&c->d_ss, c->lay.total(1) * sizeof(int2), c->stream);
   if (e == cudaSuccess && c->mi) e = dev_alloc((void**)&c->d_sbin, c->nv, c->stream);
   if (e == cudaSuccess && !cfg->high_res_is_moving && !c->mi)
     e = dev_alloc((void**)&c->d_fq, 2 * c->nv * sizeof(int), c->stream);
@@ -1706,8 +1720,8 @@ int static_sums(lc2_context* c, const TU* u) {
   ++c->launches;
   if (c->quad) {
     const size_t first = c->lay.first() + c->lay.origin();
-    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.volume() * sizeof(int), c->stream));
-    LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.volume() * sizeof(int2), c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.total(1) * sizeof(int), c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_ss, 0, c->lay.total(1) * sizeof(int2), c->stream));
     lc2::k_pad<<<blocks, 256, 0, c->stream>>>(quantised, nx, ny, nv, c->d_uq + first, c->lay.px,
                                               c->lay.slice());
     lc2::k_pad_static<<<blocks, 256, 0, c->stream>>>(c->d_sigma, c->d_su, nx, ny, nv, c->d_ss + first,
@@ -1737,7 +1751,7 @@ int fixed_static_sums(lc2_context* c) {
   lc2::k_fixed_quant<<<blocks, 256, 0, c->stream>>>((const float*)c->d_static, c->d_gstatic, nv,
                                                     c->fp.qm, c->fp.qg, c->d_fq, c->d_fd);
   if (c->quad) {
-    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, 2 * c->lay.volume() * sizeof(int), c->stream));
+    LC2_CUDA(cudaMemsetAsync(c->d_uq, 0, c->lay.total(2) * sizeof(int), c->stream));
     for (int f = 0; f < 2; ++f)
       lc2::k_pad<<<blocks, 256, 0, c->stream>>>(
           lc2::BoxImage<int>{c->d_fq + f * nv}, nx, ny, nv,

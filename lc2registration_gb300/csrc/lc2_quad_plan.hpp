@@ -9,24 +9,31 @@ namespace lc2 {
 // Presampled images and the static ultrasound's fields in the layout
 // k_fused_quad reads: every image has a border of zeros wide enough for the
 // halo and the Sobel margin of every tile, so the kernel's loads need no bounds
-// test. All have the same strides, so one offset addresses them all.
+// test. All have the same strides, so one offset addresses them all. The border
+// after a row, a slice or an image is the one before the next: a read beyond the
+// end of one lands there (at 96^3, radius 3, 1.17 times the grid's voxels; with
+// borders of their own 1.73 times).
 struct PadLayout {
-  int px, py, pz;   // padded extents (px: row pitch)
+  int px, py, pz;   // strides: voxels per row, rows per slice, slices per image
   int b;            // border voxels before x = 0, y = 0 and z = 0
   size_t slice() const { return (size_t)px * py; }
-  size_t volume() const { return slice() * pz; }
+  size_t volume() const { return slice() * pz; }  // from one image to the next
   size_t first() const { return slice() * b; }          // of slice 0
   size_t origin() const { return (size_t)px * b + b; }  // of voxel (0, 0) in a slice
+  // of n images: the border before the first, and the rows a read of the last
+  // image's last slice runs on into
+  size_t total(int n) const { return first() + volume() * n + slice(); }
 };
 
-// Border r + 1 before, and after the last tile (x: whole 32-column tiles; y:
-// the last row any tile's quads touch); z: slices -r-1 .. vz+r+1.
+// Reads of tiles of 24 and 16 rows at radius r: columns -r-1 .. 32 ntx + r, rows
+// -r-1 .. rows + r, 2 more at odd radii (whole quads of the halo), where `rows`
+// of 24-row tiles cover the grid, slices -r-1 .. vz+r+1.
 inline PadLayout pad_layout(int vx, int vy, int vz, int r) {
   PadLayout L;
   L.b = r + 1;
-  L.px = (((vx + 31) / 32 * 32 + 2 * (r + 1)) + 7) / 8 * 8;
-  L.py = (vy + 31) + 2 * (r + 1) + 4;  // tiles of at most 32 rows, whole quads
-  L.pz = vz + 2 * r + 4;
+  L.px = ((vx + 31) / 32 * 32 + L.b + 3) / 4 * 4;
+  L.py = (vy + 23) / 24 * 24 + 2 * (r & 1) + L.b;
+  L.pz = vz + 1 + L.b;
   return L;
 }
 

@@ -66,3 +66,29 @@ def test_set_images_takes_no_more_than_one_image():
         held, peak = _bytes(mode, fdim, mdim, vs, r, hr, storage)
         _, extra = _admitted(mode, fdim, mdim, vdim, r, hr, storage)
         assert peak - held <= extra, (mode, fdim, mdim, vs, r, hr, storage)
+
+
+def test_a_context_holds_no_more_than_it_was_admitted_with():
+    """But for 32 MiB of presampled images of small grids, the error flag's 4
+    bytes, and grids whose static fields and one presampled image alone are more:
+    beyond 500^3, or of a few voxels along an axis."""
+    more = 0
+    for mode, fdim, mdim, vdim, vs, r, hr, storage in _configs(600, 2):
+        held, _ = _bytes(mode, fdim, mdim, vs, r, hr, storage)
+        want, _ = _admitted(mode, fdim, mdim, vdim, r, hr, storage)
+        nv = int(np.prod(vdim))
+        quad = mode == "3D" and 1 <= r <= 4
+        if quad and (nv > 100_000_000 or min(vdim) < 8):
+            continue
+        assert held <= want + 4 + (32 << 20 if quad and 256 * nv < 32 << 20 else 0), (
+            mode, fdim, mdim, vs, r, hr, storage, held, want)
+        more += held > want + 4
+    assert more < 60
+
+
+@pytest.mark.parametrize("dim,r", [((96, 96, 96), 3), ((256, 256, 256), 4), ((160, 160, 160), 3),
+                                   ((200, 200, 8), 4), ((512, 512, 16), 4)])
+@pytest.mark.parametrize("hr_moving", [True, False])
+def test_padded_grids_fit_what_was_admitted(dim, r, hr_moving):
+    held, _ = _bytes("3D", dim, dim, [1.0] * 3, r, hr_moving, "f32")
+    assert held <= _admitted("3D", dim, dim, dim, r, hr_moving, "f32")[0] + 4

@@ -23,3 +23,15 @@ def test_plans_equal_the_full_search(tmp_path):
     assert int(bad) == 0, out
     assert int(two) > 1000, out
     assert float(planned) * 4 < float(searched), out
+
+
+def test_padded_layout_covers_every_read(tmp_path):
+    """Borders shared by neighbouring rows, slices and images: a read outside the
+    grid finds a zero, inside the allocation."""
+    if shutil.which("g++") is None:
+        pytest.skip("g++ missing")
+    exe = str(tmp_path / "pad_layout")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", os.path.join(ROOT, "tests", "cpp", "pad_layout.cpp"),
+                    "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+    assert re.match(r"0 wrong of \d{7,}", out), out
