@@ -1182,8 +1182,9 @@ const char* lc2_version(void) { return "lc2-gb300 0.1 (sm_103a)"; }
 namespace {
 
 // Host-side plan of a context: validation, virtual grid, sizes, patch and
-// fixed-point bits, scratch slots. No device work.
-int plan_context(const lc2_config* cfg, lc2_context* c) {
+// fixed-point bits, scratch slots. No device work. lean: without the padded
+// layout (16-row tiles, the same values).
+int plan_context(const lc2_config* cfg, lc2_context* c, bool lean = false) {
   if (cfg->mode < LC2_MODE_2D || cfg->mode > LC2_MODE_2DTO3D)
     return fail(LC2_ERR_INVALID_ARGUMENT, "unknown mode %d", cfg->mode);
   if (cfg->storage < LC2_STORE_F32 || cfg->storage > LC2_STORE_BF16)
@@ -1264,7 +1265,7 @@ int plan_context(const lc2_config* cfg, lc2_context* c) {
   // 3D contexts of a resampled MR/CT resample in a pass of their own
   c->presample = (c->lc2_nd == 3 && !c->mi) ? 1 : 0;
   // the padded images of k_fused_quad index a slice with 32-bit byte offsets
-  if (c->presample && r <= 4) {
+  if (c->presample && r <= 4 && !lean) {
     c->lay = lc2::pad_layout(c->virt.dim[0], c->virt.dim[1], c->virt.dim[2], r);
     c->quad = c->lay.slice() < (size_t)1 << 28;  // 16-byte fields at 32-bit offsets
   }
@@ -1297,12 +1298,12 @@ void context_bytes(const lc2_context* c, size_t* held, size_t* peak_extra) {
   if (!hrm && !c->mi) *peak_extra = std::max(*peak_extra, c->nv * sizeof(long long));
 }
 
-int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
+int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out, bool lean = false) {
   if (!cfg || !out) return fail(LC2_ERR_INVALID_ARGUMENT, "null config or output pointer");
   *out = nullptr;
   lc2_context* c = new (std::nothrow) lc2_context();
   if (!c) return fail(LC2_ERR_OUT_OF_MEMORY, "host allocation failed");
-  int st = plan_context(cfg, c);
+  int st = plan_context(cfg, c, lean);
   if (st == LC2_OK) st = select_device(c);
   if (st != LC2_OK) {
     delete c;
@@ -1366,22 +1367,30 @@ int create_context(const lc2_config* cfg, bool own_moving, lc2_context** out) {
 
 }  // namespace
 
-extern "C" {
-
-int lc2_create(const lc2_config* cfg, lc2_context** out) {
+// The server's (lc2_serve.cpp): a context as lc2_create makes it or, for a request
+// that only fits its budget so, a lean one.
+int lc2_create_as(const lc2_config* cfg, bool lean, lc2_context** out) {
   g_err.clear();
-  return create_context(cfg, true, out);
+  return create_context(cfg, true, out, lean);
 }
 
-int lc2_context_bytes(const lc2_config* cfg, size_t* held, size_t* peak) {
+int lc2_context_bytes_as(const lc2_config* cfg, bool lean, size_t* held, size_t* peak) {
   g_err.clear();
   if (!cfg || !held) return fail(LC2_ERR_INVALID_ARGUMENT, "null argument");
   lc2_context c;
-  LC2_TRY(plan_context(cfg, &c));
+  LC2_TRY(plan_context(cfg, &c, lean));
   size_t extra = 0;
   context_bytes(&c, held, &extra);
   if (peak) *peak = *held + extra;
   return LC2_OK;
+}
+
+extern "C" {
+
+int lc2_create(const lc2_config* cfg, lc2_context** out) { return lc2_create_as(cfg, false, out); }
+
+int lc2_context_bytes(const lc2_config* cfg, size_t* held, size_t* peak) {
+  return lc2_context_bytes_as(cfg, false, held, peak);
 }
 
 int lc2_destroy(lc2_context* c) {

@@ -29,7 +29,10 @@
 
 #include "../../include/lc2.h"
 
+// lc2_capi.cu
 void lc2_set_error_message(const char* msg);
+int lc2_create_as(const lc2_config* cfg, bool lean, lc2_context** out);
+int lc2_context_bytes_as(const lc2_config* cfg, bool lean, size_t* held, size_t* peak);
 
 namespace {
 
@@ -56,6 +59,7 @@ struct Job {
   std::vector<lc2_registration> frame_regs;
   std::vector<lc2_request_result> frame_res;
   size_t bytes = 0;
+  bool lean = false;  // its context without padded images: the budget holds no other
   enum { Queued, Running, Done } state = Queued;
   lc2_request_result res{};
   Clock::time_point t_submit, t_admit, t_done;
@@ -236,7 +240,7 @@ struct lc2_server {
       lc2_context* c = nullptr;
       lc2_config cfg = j.req.config;
       cfg.device = this->cfg.device;
-      st = lc2_create(&cfg, &c);
+      st = lc2_create_as(&cfg, j.lean, &c);
       // small requests (virtual grid up to 2^20 voxels) on the most urgent
       // stream priority: their short launches are scheduled ahead of the
       // CTAs of large concurrent ones
@@ -398,6 +402,9 @@ int lc2_server_submit(lc2_server* s, const lc2_request* req, long long* ticket) 
   const bool host_objective = req->registration.lc2_of_matrices != nullptr;
   if (!host_objective && (!req->fixed || !req->moving))
     return fail(LC2_ERR_INVALID_ARGUMENT, "request without images");
+  const bool lean = peak > s->cfg.hbm_budget_bytes;
+  if (lean) st = lc2_context_bytes_as(&cfg, true, &held, &peak);
+  if (st != LC2_OK) return st;
   if (peak > s->cfg.hbm_budget_bytes)
     return fail(LC2_ERR_OUT_OF_MEMORY, "request needs " + std::to_string(peak) +
                                            " device bytes, the budget is " +
@@ -405,6 +412,7 @@ int lc2_server_submit(lc2_server* s, const lc2_request* req, long long* ticket) 
   auto j = std::make_shared<Job>();
   j->req = *req;
   j->bytes = peak;
+  j->lean = lean;
   if (!host_objective) {
     const bool flat = cfg.mode == LC2_MODE_2D;
     j->fixed.assign(req->fixed, req->fixed + image_voxels(cfg.fixed, flat));

@@ -50,3 +50,38 @@ def test_peak_is_not_exceeded(dim, r, hr_moving):
             ctx.evaluate_batch(np.stack([mat] * 64))
     ctx.close()
     assert held / 2 < w.top <= peak
+
+
+@pytest.mark.parametrize("hr_moving", [True, False])
+def test_request_without_padded_fields_equals_alone(hr_moving):
+    """A budget that holds a request's context only without its padded fields:
+    the same registration as with them."""
+    from lc2registration_gb300 import synth
+    from tests.helpers import make_context
+    from tests.test_memory_plan import _admitted
+
+    case = synth.case_3d(seed=14, mr_size=32, us_size=24, r=2, blobs=6)
+    if not hr_moving:
+        case = synth.Case("3D", case.moving_geom, case.moving, case.fixed_geom, case.fixed,
+                          list(case.moving_geom.spacing), 2, hr_moving=False, true_params={}, true_mat=None)
+    c = case.fixed_geom.center()
+    reg = dict(initial=[0, 0, 0, 0, 0, 0, 1, 1, 1, 0, 0, 0],
+               lower=[-8, -8, -8, -6, -6, -6] + [0.9] * 3 + [-0.05] * 3,
+               upper=[8, 8, 8, 6, 6, 6] + [1.1] * 3 + [0.05] * 3, center=c,
+               direct_entries=["translation"], direct_maxeval=40, rounds=[(["translation", "rotation"], 1e-3)])
+    ctx = make_context(case)
+    alone = capi.register(ctx, **reg)
+    held, extra = _admitted("3D", case.fixed_geom.dim, case.moving_geom.dim, ctx.virtual_dims(), 2,
+                            hr_moving, "f32")
+    ctx.close()
+    cfg = capi.make_config("3D", case.fixed_geom, case.moving_geom, case.virt_spacing, 2, hr_moving)
+    budget = held + 4 + extra
+    assert capi.context_bytes(cfg)[1] > budget
+    srv = capi.Server(budget_bytes=budget, max_active=2)
+    with Watch() as w:
+        got = srv.poll(srv.submit(cfg, case.fixed, case.moving, **reg))
+    srv.close()
+    assert got["status"] == 0, got["message"]
+    np.testing.assert_array_equal(got["params"][:12], alone["params"])
+    assert got["lc2"] == alone["lc2"] and got["evaluations"] == alone["evaluations"]
+    assert w.top <= budget

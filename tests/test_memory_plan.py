@@ -92,3 +92,27 @@ def test_a_context_holds_no_more_than_it_was_admitted_with():
 def test_padded_grids_fit_what_was_admitted(dim, r, hr_moving):
     held, _ = _bytes("3D", dim, dim, [1.0] * 3, r, hr_moving, "f32")
     assert held <= _admitted("3D", dim, dim, dim, r, hr_moving, "f32")[0] + 4
+
+
+def test_server_takes_every_request_that_fits_without_padded_fields():
+    """Small, thin and very large grids whose padded fields pass the budget run
+    without them; one byte less is refused."""
+    reg = dict(initial=[0, 0, 0, 0, 0, 0, 1, 1, 1, 0, 0, 0], lower=[-1] * 6 + [0.9] * 3 + [-0.1] * 3,
+               upper=[1] * 6 + [1.1] * 3 + [0.1] * 3, center=(8.0, 8.0, 8.0),
+               rounds=[(["translation"], 1e-2)])
+    geo = lambda d: Geometry(d, (1.0, 1.0, 1.0), (0.0, 0.0, 0.0))
+    for dim, r in (((16, 16, 16), 2), ((24, 20, 1), 4), ((2, 218, 474), 4), ((600, 500, 700), 4)):
+        for hr in (True, False):
+            cfg = capi.make_config("3D", geo(dim), geo(dim), [1.0] * 3, r, hr)
+            held, extra = _admitted("3D", dim, dim, dim, r, hr, "f32")
+            lean = held + 4 + (4 * int(np.prod(dim)) if hr else 8 * int(np.prod(dim)))
+            assert capi.context_bytes(cfg)[1] > lean
+            srv = capi.Server(budget_bytes=lean, max_active=1)
+            t = srv.submit(cfg, lc2_of_matrices=lambda m: np.ones(len(m)), **reg)
+            assert srv.poll(t)["status"] == 0
+            assert srv.stats()["peak_bytes"] == lean <= held + 4 + extra
+            srv.close()
+            srv = capi.Server(budget_bytes=lean - 1, max_active=1)
+            with pytest.raises(capi.LC2Error, match="OUT_OF_MEMORY"):
+                srv.submit(cfg, lc2_of_matrices=lambda m: np.ones(len(m)), **reg)
+            srv.close()
