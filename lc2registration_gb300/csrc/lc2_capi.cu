@@ -746,8 +746,8 @@ void choose_zchunks(const lc2_context* c, int cnt, lc2::MomentParams& P) {
 }
 
 // Generic path: resample -> Sobel -> moments through global scratch. Used for
-// a resampled ultrasound (HighResolutionModality: Fixed), for the one-time
-// weighting-factor precompute and for the diagnostic field dumps.
+// LC2_OPTION_GENERIC and, with a resampled ultrasound (HighResolutionModality:
+// Fixed), for the field dumps and the weighting map.
 int launch_group_generic(lc2_context* c, int k0, int cnt, float* osig, float* omeas) {
   const size_t nv = c->nv;
   lc2::MomentParams P = c->mp;
@@ -834,8 +834,10 @@ int presample_cap(const lc2_context* c, bool padded) {
 // voxels of the grid only.
 int ensure_presample(lc2_context* c, int count) {
   const bool padded = use_quad(c);
+  const bool same = c->d_pre && c->pre_padded == padded;
+  if (same && c->pre_slots >= count) return LC2_OK;
   const int want = std::max(1, std::min(count, presample_cap(c, padded)));
-  if (c->d_pre && c->pre_slots >= want && c->pre_padded == padded) return LC2_OK;
+  if (same && c->pre_slots >= want) return LC2_OK;
   drop_graphs(c);
   dev_free(c->d_pre, c->stream);
   c->d_pre = nullptr;

@@ -35,13 +35,13 @@ constexpr int list_rows(int r) { return r <= 6 ? 32 : 16; }
 
 template <int R, bool QUAD = (R <= 6)>
 struct ListGeom {
-  static constexpr int TY = list_rows(R), NT = 32 * TY, CTAS = 3, ST = NT;
+  static constexpr int TY = list_rows(R), NT = 32 * TY, CTAS = 3;
   static constexpr size_t BYTES = FusedGeom<2, TY, R>::BYTES;
 };
 template <int R>
 struct ListGeom<R, true> {
   using G = Quad2D<list_rows(R), R>;
-  static constexpr int TY = list_rows(R), NT = G::NT, CTAS = G::CTAS, ST = G::ST;
+  static constexpr int TY = list_rows(R), NT = G::NT, CTAS = G::CTAS;
   static constexpr size_t BYTES = G::BYTES;
 };
 

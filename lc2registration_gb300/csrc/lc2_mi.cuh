@@ -7,18 +7,18 @@
 // histogram indexed ultrasound bin + 256 * high-resolution bin.
 //
 // One image is static (the fixed one resampled once): its bins and entropy
-// are computed once per context. Per batch of transforms four kernels run:
-// the range of the warped image (ordered-integer atomics, one pair per CTA),
-// the joint histogram (warp-aggregated integer atomics into a 256 KB
-// histogram per transform, which stays in L2), the entropy sums of slices of
+// are computed once per context, by kernels of their own. Per batch of transforms
+// four kernels run: the range of the warped image (ordered-integer atomics, one
+// pair per CTA), the joint histogram (all its bins in shared memory, added to
+// the transform's 256 KB histogram at the end), the entropy sums of slices of
 // each histogram (kMiParts CTAs per transform) and their combination in a
-// fixed order. The range and histogram CTAs each own a 32 x 8 tile over a
-// chunk of kMiChunk slices: the tile's sampling bases for all its slices are
-// computed up front, one per thread, so the slices then stream without
-// barriers; the bases are those of the generic warp kernel (tile_base), so
-// the warped values are bit-identical to it. Counts are exact integers and
-// the double sums run in a fixed order, so the value does not depend on the
-// launch shape or the batch.
+// fixed order. A range CTA owns a 32 x 8 tile over a chunk of slices, a
+// histogram CTA takes 32 x 32 x 32 blocks in turn: the sampling bases of a
+// chunk's or block's slices are computed up front, one per thread, so the slices
+// then stream without barriers; the bases are those of the generic warp kernel
+// (tile_base), so the warped values are bit-identical to it. Counts are exact
+// integers and the double sums run in a fixed order, so the value does not
+// depend on the launch shape or the batch.
 #pragma once
 
 #include "lc2_kernels.cuh"
@@ -46,8 +46,8 @@ __device__ __forceinline__ float mi_unord(unsigned u) {
 
 // Bin of v in [lo, hi]: round((v - lo) * (255 / (hi - lo))) with float
 // operations rounded to nearest (cu_lc2_3d.cu:886-889, 913); all voxels go
-// to bin 0 when hi == lo. The host computes the static image's bins with the
-// same operations.
+// to bin 0 when hi == lo. The static image's bins take the same operations
+// (k_mi_static_bins).
 __host__ __device__ inline float mi_scale(float lo, float hi) {
   return hi > lo ? 255.0f / (hi - lo) : 0.0f;
 }
