@@ -115,7 +115,8 @@ int lc2_evaluate_batch(lc2_context* ctx, const float* matrices, int count, doubl
 /* Asynchronous pieces of lc2_evaluate_batch, for callers that time or
  * overlap the device work: stage copies the matrices to the device, launch
  * enqueues every kernel on the context stream, fetch copies results back and
- * synchronises the stream. */
+ * synchronises the stream. After lc2_evaluate(_batch) the transforms evaluated
+ * are the staged ones and their values can be fetched. */
 int lc2_stage_transforms(lc2_context* ctx, const float* matrices, int count);
 int lc2_launch_staged(lc2_context* ctx, int count);
 int lc2_fetch_results(lc2_context* ctx, double* lc2_out, int count);
@@ -200,9 +201,9 @@ enum { LC2_OPTION_GENERIC = 7 };
 /* LC2_OPTION_PRESAMPLE (3D, HighResolutionModality Moving): how the moving
  * image is resampled. 1 (the default of such contexts): in a pass of its own,
  * one float per virtual voxel and transform written to a context buffer that
- * grows with the batch up to 2 GiB (25 transforms at 256^3; larger batches
- * run in groups), which the fused kernel then reads; 0: inside the fused
- * kernel. Other values are refused (LC2_ERR_INVALID_ARGUMENT). Each voxel is
+ * grows with the batch until it and the context's padded fields take 2 GiB
+ * (25 transforms at 256^3; larger batches run in groups), which the fused
+ * kernel then reads; 0: inside the fused kernel. Other values are refused (LC2_ERR_INVALID_ARGUMENT). Each voxel is
  * sampled once from its 32 x 8 tile's base in form 1 and from the fused
  * tile's base in form 0, so 0 and 1 agree to FP32 resampling rounding (about
  * 1e-7 relative on LC2), not bit for bit. Within a form no option changes a
@@ -406,7 +407,8 @@ typedef struct {
 int lc2_context_bytes(const lc2_config* cfg, size_t* held, size_t* peak);
 int lc2_server_create(const lc2_server_config* cfg, lc2_server** out);
 /* Queues a request; *ticket identifies it. LC2_ERR_OUT_OF_MEMORY when the
- * request alone exceeds the budget. */
+ * request alone exceeds the budget, for a 3D request also without the padded
+ * fields that lc2_context_bytes counts. */
 int lc2_server_submit(lc2_server* s, const lc2_request* req, long long* ticket);
 /* Queues a stack request; polled with lc2_server_poll_stack. */
 int lc2_server_submit_stack(lc2_server* s, const lc2_stack_request* req, long long* ticket);

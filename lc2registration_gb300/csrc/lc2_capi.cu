@@ -1696,8 +1696,8 @@ void box_z(lc2_context* c, const T* in, T* out) {
 // Static ultrasound: its window sums S_U, weighting factors and their sum, by
 // exact box sums in the buffers the context holds: scratch slot 0 and d_sigma
 // with d_su behind it are eight bytes per voxel each. With it, the checks on the
-// device and the fixed image through k_presample, lc2_set_images takes 24.5 ->
-// 1.6 ms on 256^3 host volumes and 2.3 -> 0.29 ms for 128^3 -> 96^3 (the generic
+// device and the fixed image through k_presample, lc2_set_images takes 24.2 ->
+// 1.5 ms on 256^3 host volumes and 1.44 -> 0.23 ms on 96^3 (at 256^3 the generic
 // moments kernel alone took 1.4, line-by-line sums 0.4 and the host's scan for
 // NaN about 20 ms).
 template <typename TU>
