@@ -1664,6 +1664,19 @@ struct TempBuffer {
   ~TempBuffer() { free(); }
 };
 
+// Waits for the stream when a call that reads the caller's images fails half-way:
+// they are the caller's again on every return.
+struct DrainOnError {
+  cudaStream_t st;
+  int done(int status) {
+    if (status == LC2_OK) st = nullptr;  // the call has waited itself
+    return status;
+  }
+  ~DrainOnError() {
+    if (st) cudaStreamSynchronize(st);
+  }
+};
+
 // The passes of window sums over the context's patch, out of place: along x from
 // any source, along y, along z.
 template <typename T, typename In>
@@ -1948,6 +1961,7 @@ int lc2_set_images(lc2_context* c, const float* fixed, const float* moving) {
   if (!c->owns_moving)
     return fail(LC2_ERR_INVALID_ARGUMENT, "the frames of a stack share the stack's moving volume");
   LC2_TRY(select_device(c));
+  DrainOnError drain{c->stream};
   // one image at a time to the device, where it is checked; the context's own
   // images stay until both are found good
   float mx[2];
@@ -1970,7 +1984,7 @@ int lc2_set_images(lc2_context* c, const float* fixed, const float* moving) {
   c->ready = false;
   LC2_TRY(convert_to_storage(c, m.p, c->d_moving, c->nm, c->cfg.storage));
   m.free();
-  return set_fixed(c, mx[0], mx[1]);
+  return drain.done(set_fixed(c, mx[0], mx[1]));
 }
 
 int lc2_set_images_device(lc2_context* c, const float* fixed, const float* moving) {
@@ -1989,6 +2003,7 @@ int lc2_set_images_device(lc2_context* c, const float* fixed, const float* movin
                   "lc2_set_images_device needs device memory of the context's device");
     }
   }
+  DrainOnError drain{c->stream};
   float mx[2];
   bool bad[2];
   LC2_TRY(absmax_clear(c));
@@ -2000,7 +2015,7 @@ int lc2_set_images_device(lc2_context* c, const float* fixed, const float* movin
   c->ready = false;
   LC2_TRY(sample_fixed(c, fixed));
   LC2_TRY(convert_to_storage(c, moving, c->d_moving, c->nm, c->cfg.storage));
-  return set_fixed(c, mx[0], mx[1]);
+  return drain.done(set_fixed(c, mx[0], mx[1]));
 }
 
 }  // extern "C"
