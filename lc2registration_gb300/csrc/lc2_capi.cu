@@ -197,6 +197,8 @@ struct lc2_context {
   double* h_out = nullptr;     // pinned results
   int staged = 0;              // transforms of the last stage or evaluation, in h_xf
   bool xf_stale = false;       // they are not in d_xf (upload_staged)
+  bool uploading = false;      // an upload may still read h_xf, until this event
+  cudaEvent_t uploaded = nullptr;
 
   lc2::MomentParams mp{};
   lc2::FusedParams fp{};
@@ -1430,6 +1432,7 @@ int lc2_destroy(lc2_context* c) {
     cudaEventDestroy(t.a);
     cudaEventDestroy(t.b);
   }
+  if (c->uploaded) cudaEventDestroy(c->uploaded);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
   return LC2_OK;
@@ -2035,6 +2038,8 @@ int stage_host(lc2_context* c, const float* matrices, int count) {
   LC2_TRY(ensure_capacity(c, count));
   if (c->presample && !c->generic && !(c->pipeline && c->cfg.high_res_is_moving))
     LC2_TRY(ensure_presample(c, count));
+  if (c->uploading) LC2_CUDA(cudaEventSynchronize(c->uploaded));
+  c->uploading = false;
   for (int k = 0; k < count; ++k)
     build_xform(c->warp_nd, c->virt, c->cfg.moving, matrices + (size_t)k * mf, &c->h_xf[k]);
   c->staged = count;
@@ -2042,11 +2047,20 @@ int stage_host(lc2_context* c, const float* matrices, int count) {
   return LC2_OK;
 }
 
-// The staged transforms into d_xf, if they are on the host only.
+// The staged transforms into d_xf, if they are on the host only. The copy waits
+// for the stream's earlier work, and the next stage for the copy.
 int upload_staged(lc2_context* c) {
-  if (c->staged > 0 && c->xf_stale)
+  if (c->staged > 0 && c->xf_stale) {
     LC2_CUDA(cudaMemcpyAsync(c->d_xf, c->h_xf, sizeof(lc2::Xform) * c->staged,
                              cudaMemcpyHostToDevice, c->stream));
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    LC2_CUDA(cudaStreamIsCapturing(c->stream, &capturing));
+    if (capturing == cudaStreamCaptureStatusNone) {
+      if (!c->uploaded) LC2_CUDA(cudaEventCreateWithFlags(&c->uploaded, cudaEventDisableTiming));
+      LC2_CUDA(cudaEventRecord(c->uploaded, c->stream));
+      c->uploading = true;
+    }
+  }
   c->xf_stale = false;
   return LC2_OK;
 }

@@ -96,3 +96,21 @@ def test_staged_launch_does_not_pay_for_larger_batches():
     ctx.evaluate_batch(mats)
     assert one() < before + 60e-6
     ctx.close()
+
+
+def test_staging_ahead_of_a_running_launch():
+    """Transforms staged while an earlier launch runs: the copy of the ones
+    before them has read them by then."""
+    case = synth.case_3d(seed=6, mr_size=64, us_size=64, r=3, blobs=5)
+    a, b, c = (perturbed(case, np.random.default_rng(s), 200) for s in (1, 2, 3))
+    ctx = make_context(case)
+    want = ctx.evaluate_batch(b)
+    for _ in range(5):
+        ctx.stage(a)
+        for _ in range(4):
+            ctx.launch(200)
+        ctx.stage(b)
+        ctx.launch(200)
+        ctx.stage(c)
+        np.testing.assert_array_equal(ctx.fetch(200), want)
+    ctx.close()
