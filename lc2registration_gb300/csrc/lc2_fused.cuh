@@ -408,7 +408,7 @@ __device__ __forceinline__ float fused_sobel_sd(const float2* SD, int c) {
 // whether the region lies in the virtual grid (origin gx0, gy0; zin: the
 // slice is in the grid) with every sample of it strictly inside the moving
 // image along its first WND axes (0 <= floor, floor + 1 <= dim - 1; the
-// region's corners bound the affine image within the limits of region_end).
+// region's corners bound the affine image within the limits of before_end).
 template <int WND, int PW, int PH>
 __device__ __forceinline__ bool region_base(const Xform& X, const float* A, const FusedParams& P,
                                             int gx0, int gy0, int yb, int zs, bool zin,
@@ -424,7 +424,7 @@ __device__ __forceinline__ bool region_base(const Xform& X, const float* A, cons
       const float lo = fb[a] + fminf(ex, 0.0f) + fminf(e0, e1);
       const float hi = fb[a] + fmaxf(ex, 0.0f) + fmaxf(e0, e1);
       in = in && ((float)ib[a] + lo >= 0.01f) &&
-           ((float)ib[a] + hi <= region_end((float)(dims[a] - 1))) &&
+           before_end((float)ib[a] + hi, (float)(dims[a] - 1)) &&
            lo > -kRegionSpan && hi < kRegionSpan;
     }
   }

@@ -267,7 +267,9 @@ __device__ __forceinline__ float trilinear(const TM* __restrict__ mov, unsigned 
 // position rounds to 2^-24 of it, so the far end's limit gives way with the axis
 // (a fixed 0.01 voxel passes samples beyond the last voxel of axes of 10^5).
 constexpr float kRegionSpan = 4096.0f;
-__device__ __forceinline__ float region_end(float end) { return fmaf(end, 0.999999f, -0.01f); }
+__device__ __forceinline__ bool before_end(float h, float end) {
+  return h + 1e-6f * end <= end - 0.01f;
+}
 
 // Where the samples of a 32 x 8 tile slice from base T lie: strictly inside the
 // moving volume (0 <= floor, floor + 1 <= dim - 1 on each axis), all outside
@@ -283,7 +285,7 @@ __device__ __forceinline__ int tile_where(const TileBase& T, int mx, int my, int
     const float lo = T.fb[a] + fminf(ex, 0.0f) + fminf(ey, 0.0f);
     const float hi = T.fb[a] + fmaxf(ex, 0.0f) + fmaxf(ey, 0.0f);
     const float l = (float)T.ib[a] + lo, h = (float)T.ib[a] + hi, end = (float)(dims[a] - 1);
-    in = in && (l >= 0.01f) && (h <= region_end(end));
+    in = in && (l >= 0.01f) && before_end(h, end);
     out = out || (h < -0.01f - 1e-6f * fabsf(h)) || (l > end + 0.01f + 1e-6f * end);
     near = near && (lo > -kRegionSpan) && (hi < kRegionSpan);
   }
